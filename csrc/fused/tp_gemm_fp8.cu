@@ -13,6 +13,7 @@
 #include "sm100_ptx.cuh"
 #include "tp_gemm.cuh"
 #include "tp_device.cuh"
+#include "tp_skinny.cuh"
 
 namespace xccl {
 namespace tp {
@@ -44,6 +45,11 @@ using namespace xccl::tp;
 extern "C" xccl_status_t xccl_gemm_fp8_blockscaled(const void *A8, const float *sa, const void *B8, const float *sb, void *C,
                                                    int M, int N, int K, void *stream)
 {
+    SkinnyArgs    sk{};
+    xccl_status_t sst;
+    sk.M = M; sk.N = N; sk.K = K; sk.fp8 = true;
+    sk.A = A8; sk.B0 = B8; sk.C = C; sk.ldc = N; sk.sa = sa; sk.sb0 = sb;
+    if (try_skinny(sk, (cudaStream_t)stream, &sst)) return sst;
     GemmParams p{};
     GemmLaunch l{};
     p.M = M; p.N = N; p.K = K;

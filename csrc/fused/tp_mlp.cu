@@ -18,6 +18,7 @@
 #include "../tl/nvlink/nvl_shm.h"
 #include "tp_gemm.cuh"
 #include "tp_mlp.h"
+#include "tp_skinny.cuh"
 
 namespace xccl {
 namespace tp {
@@ -235,6 +236,13 @@ xccl_status_t xccl_tp_ag_gemm_swiglu(xccl_tp_ws_h w, const void *const *Wg, cons
     if (w == nullptr || Wg == nullptr || Wu == nullptr || Hout == nullptr || F_local % (kBN / 2) != 0) {
         return XCCL_ERR_INVALID_PARAM;
     }
+    if (w->tp == 1 && !w->in_active) {  // one rank, the rows are there
+        SkinnyArgs    sk{};
+        xccl_status_t sst;
+        sk.M = w->M; sk.N = F_local; sk.K = w->K; sk.swiglu = true;
+        sk.A = w->xg(0); sk.B0 = Wg[0]; sk.B1 = Wu[0]; sk.C = Hout[0]; sk.ldc = F_local; sk.error = w->error;
+        if (try_skinny(sk, (cudaStream_t)stream, &sst)) return sst;
+    }
     GemmParams p{};
     GemmLaunch l{};
     p.M = w->M;
@@ -340,6 +348,13 @@ xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void
                               int F_local, void *stream)
 {
     if (w == nullptr || Hin == nullptr || Wd == nullptr || Yout == nullptr || F_local % 8 != 0) return XCCL_ERR_INVALID_PARAM;
+    if (w->tp == 1) {
+        SkinnyArgs    sk{};
+        xccl_status_t sst;
+        sk.M = w->M; sk.N = w->N_rs; sk.K = F_local;
+        sk.A = Hin[0]; sk.B0 = Wd[0]; sk.C = Yout[0]; sk.ldc = w->N_rs; sk.error = w->error;
+        if (try_skinny(sk, (cudaStream_t)stream, &sst)) return sst;
+    }
     GemmParams p{};
     GemmLaunch l{};
     p.M = w->M;
@@ -422,6 +437,14 @@ xccl_status_t xccl_tp_ag_gemm_swiglu_fp8q(xccl_tp_ws_h w, const void *const *Wg8
         F_local % 128 != 0 || w->K % 128 != 0) {
         return XCCL_ERR_INVALID_PARAM;
     }
+    if (w->tp == 1) {
+        SkinnyArgs    sk{};
+        xccl_status_t sst;
+        sk.M = w->M; sk.N = F_local; sk.K = w->K; sk.fp8 = true; sk.swiglu = true;
+        sk.A = w->xg(0); sk.B0 = Wg8[0]; sk.B1 = Wu8[0]; sk.C = Hout[0]; sk.ldc = F_local; sk.error = w->error;
+        sk.sa = w->sx(0); sk.sb0 = sWg[0]; sk.sb1 = sWu[0]; sk.out_scale = out_scales != nullptr ? out_scales[0] : nullptr;
+        if (try_skinny(sk, (cudaStream_t)stream, &sst)) return sst;
+    }
     GemmParams p{};
     GemmLaunch l{};
     p.M = w->M;
@@ -472,6 +495,14 @@ xccl_status_t xccl_tp_gemm_rs_fp8(xccl_tp_ws_h w, const void *const *H8, const f
     if (w == nullptr || H8 == nullptr || sH == nullptr || Wd8 == nullptr || sWd == nullptr || Yout == nullptr ||
         F_local % 128 != 0 || w->N_rs % 128 != 0) {
         return XCCL_ERR_INVALID_PARAM;
+    }
+    if (w->tp == 1) {
+        SkinnyArgs    sk{};
+        xccl_status_t sst;
+        sk.M = w->M; sk.N = w->N_rs; sk.K = F_local; sk.fp8 = true;
+        sk.A = H8[0]; sk.B0 = Wd8[0]; sk.C = Yout[0]; sk.ldc = w->N_rs; sk.error = w->error;
+        sk.sa = sH[0]; sk.sb0 = sWd[0];
+        if (try_skinny(sk, (cudaStream_t)stream, &sst)) return sst;
     }
     GemmParams p{};
     GemmLaunch l{};

@@ -1,0 +1,45 @@
+"""How the few-rows GEMM cuts its work (``csrc/fused/tp_skinny.cu``), walked on the CPU."""
+import ctypes as C
+
+import pytest
+
+from xccl_b200 import _capi as K
+
+FIELDS = ("mn", "tiles", "splits", "kblocks", "stages", "nbuf", "cols", "tmem_cols", "chunk", "smem", "occ")
+
+
+def _plan(M, N, K_, fp8, swiglu, sms=148):
+    out = (C.c_int * len(FIELDS))()
+    fn = K.load().xccl_tp_skinny_plan
+    fn.restype = C.c_int
+    return dict(zip(FIELDS, out)) if fn(M, N, K_, int(fp8), int(swiglu), sms, out) else None
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_plan_covers_the_product_and_fits_the_sm(fp8, swiglu):
+    for M in list(range(1, 129)):
+        for N in (8, 128, 1000, 8192, 28672, 60000):
+            for K_ in (8, 128, 520, 8192, 28672):
+                if fp8 and (K_ % 128 or N % 128):
+                    continue
+                p = _plan(M, N, K_, fp8, swiglu)
+                assert p is not None
+                mats = 2 if swiglu else 1
+                assert M <= p["mn"] <= 128 and p["mn"] % (32 if fp8 else 16) == 0
+                assert (p["tiles"] - 1) * 128 < N <= p["tiles"] * 128
+                # every K block belongs to exactly one CTA and none is without work
+                cut = [s * p["kblocks"] // p["splits"] for s in range(p["splits"] + 1)]
+                assert 1 <= p["splits"] <= 8 and cut[-1] == p["kblocks"] and all(a < b for a, b in zip(cut, cut[1:]))
+                # shared memory and tensor memory of the CTAs that share an SM
+                assert (p["smem"] + 1024 + 64) * p["occ"] <= 228 * 1024
+                assert p["tmem_cols"] * p["occ"] <= 512 and p["nbuf"] * p["cols"] <= p["tmem_cols"]
+                assert p["tmem_cols"] & (p["tmem_cols"] - 1) == 0 and p["cols"] >= mats * p["mn"]
+                ring = p["stages"] * (16384 * mats + p["mn"] * 128)
+                assert p["stages"] >= 2 and 16 <= p["chunk"] <= p["mn"] and p["chunk"] % 16 == 0
+                assert p["chunk"] * 512 * mats <= ring
+
+
+def test_more_rows_than_one_mma_are_left_to_the_large_kernel():
+    assert _plan(129, 8192, 8192, False, False) is None
+    assert _plan(0, 8192, 8192, False, False) is None

@@ -659,6 +659,69 @@ def test_gemm_fp8_blockscaled_matches_dequantised_reference(dev, M, N, K_):
     torch.testing.assert_close(out.float(), want, rtol=2e-2, atol=2e-2 * float(want.abs().max()))
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 127, 128, 129])
+@pytest.mark.parametrize("N,K_", [(8, 8), (264, 520), (1024, 4104)])
+def test_gemm_few_rows_matches_fp32_reference(dev, M, N, K_):
+    """Row counts around the edges of the few-rows kernel (its MMA takes 16-row steps up to 128), one CTA per weight
+    tile and several that share K, ragged last tiles in N and K."""
+    from xccl_b200.ops import gemm
+    a = torch.randn(M, K_, device=dev).to(torch.bfloat16)
+    b = torch.randn(N, K_, device=dev).to(torch.bfloat16)
+    guard = torch.full((M + 2, N), 7.0, device=dev, dtype=torch.bfloat16)
+    gemm.gemm_bf16(a, b, guard[1:M + 1])
+    assert gemm.last_error() == 0
+    want = a.float() @ b.float().t()
+    # bf16 rounding of the result (2^-9 of it) and of fp32 sums of K products of size 1: far below 1e-2 of sqrt(K)
+    torch.testing.assert_close(guard[1:M + 1].float(), want, rtol=1e-2, atol=1e-2 * K_ ** 0.5)
+    assert bool((guard[0] == 7).all()) and bool((guard[M + 1] == 7).all())
+
+
+@pytest.mark.parametrize("M", [1, 33, 100, 128])
+@pytest.mark.parametrize("F,K_", [(128, 64), (384, 1000), (2048, 4096)])
+def test_gemm_swiglu_few_rows_matches_fp32_reference(dev, M, F, K_):
+    from xccl_b200.ops import gemm
+    a = torch.randn(M, K_, device=dev).to(torch.bfloat16)
+    wg = (torch.randn(F, K_, device=dev) / K_ ** 0.5).to(torch.bfloat16)
+    wu = (torch.randn(F, K_, device=dev) / K_ ** 0.5).to(torch.bfloat16)
+    out = gemm.gemm_swiglu(a, wg, wu)
+    assert gemm.last_error() == 0
+    want = torch.nn.functional.silu(a.float() @ wg.float().t()) * (a.float() @ wu.float().t())
+    torch.testing.assert_close(out.float(), want, rtol=1e-2, atol=1e-2)   # values of size 1, one bf16 rounding
+
+
+@pytest.mark.parametrize("M", [1, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K_", [(128, 128), (384, 1152), (1024, 8192)])
+def test_gemm_fp8_few_rows_matches_dequantised_reference(dev, M, N, K_):
+    from xccl_b200.ops import gemm
+    a = torch.randn(M, K_, device=dev) * torch.rand(M, 1, device=dev) * 3
+    b = torch.randn(N, K_, device=dev) * 0.05
+    a8, sa = gemm.quantize_act_1x128(a)
+    b8, sb = gemm.quantize_weight_128x128(b)
+    out = gemm.gemm_fp8_blockscaled(a8, sa, b8, sb)
+    assert gemm.last_error() == 0
+    want = gemm.dequantize(a8, sa, 1) @ gemm.dequantize(b8, sb, 128).t()
+    torch.testing.assert_close(out.float(), want, rtol=1e-2, atol=1e-2 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_tp_mlp_one_block_of_rows_matches_reference(dev, fp8):
+    """The block with 128 tokens on one rank: both products run in the few-rows kernel, in fp8 with the intermediate
+    quantised by it."""
+    from xccl_b200.models.tp_mlp import TpMlp, TpMlpFp8, reference_forward_fp32
+    mlp = (TpMlpFp8 if fp8 else TpMlp)(128, 1024, 2048, tp=1)
+    try:
+        x = torch.randn(128, 1024, device=dev).to(torch.bfloat16)
+        for _ in range(2):
+            got = mlp.forward([x])[0].float()
+            mlp.check_error()
+        want = reference_forward_fp32(x, *_full_weights(mlp))
+        # bf16: two roundings of 2^-9; fp8: 2^-4 per quantised operand, averaged over the sums
+        tol = 0.08 if fp8 else 0.02
+        assert float((got - want).abs().max()) <= tol * float(want.abs().max()) + 1e-3
+    finally:
+        mlp.close()
+
+
 def test_quantize_rows_kernel_matches_torch(dev):
     from xccl_b200.ops import gemm
     from xccl_b200.ops.tp import quantize_rows
