@@ -645,6 +645,26 @@ def test_moe_dispatch_combine_matches_reference(dev, ranks):
         ws.close()
 
 
+def test_moe_views_outlive_the_workspace(dev):
+    """A tensor on workspace memory keeps that memory after close(); without views close() frees it."""
+    from xccl_b200.ops.moe import MoeWorkspace
+    ws = MoeWorkspace(16, 64, 8, 2)
+    x = torch.randn(16, 64, device=dev).to(torch.bfloat16)
+    ids = torch.stack([torch.arange(16) % 8, (torch.arange(16) + 1) % 8], 1).to(torch.int32).to(dev)
+    ws.dispatch([x], [ids])
+    rows, recv = ws.expert_rows(), ws.recv()
+    ws.close()
+    assert rows.cpu().tolist() == [4] * 8 + [32]
+    assert float(recv.float().abs().sum()) == pytest.approx(2 * float(x.float().abs().sum()), rel=1e-3)
+    del rows, recv
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    big = MoeWorkspace(4096, 4096, 8, 4)          # 256 MB and more
+    assert torch.cuda.mem_get_info()[0] < free - (200 << 20)
+    big.close()
+    assert torch.cuda.mem_get_info()[0] > free - (64 << 20)
+
+
 # ----------------------------------------------------------------------------- block-scaled fp8 GEMM
 @pytest.mark.parametrize("M,N,K_", [(128, 128, 128), (256, 384, 512), (1000, 256, 1024), (2048, 1024, 2048)])
 def test_gemm_fp8_blockscaled_matches_dequantised_reference(dev, M, N, K_):

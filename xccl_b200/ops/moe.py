@@ -30,7 +30,19 @@ def _ptrs(ts: Sequence[torch.Tensor]):
     return arr
 
 
-def _view(ptr: int, shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
+class _Workspace:
+    """The native workspace; its memory is freed with the last reference to it."""
+
+    def __init__(self, h: C.c_void_p):
+        self.h = h
+
+    def __del__(self):
+        K.load().xccl_moe_ws_destroy(self.h)
+
+
+def _view(ptr: int, shape: tuple, dtype: torch.dtype, device, owner: _Workspace) -> torch.Tensor:
+    """A tensor on workspace memory. It keeps the workspace: the memory outlives ``MoeWorkspace.close`` for as long as a
+    view of it does."""
     n = 1
     for s in shape:
         n *= s
@@ -39,7 +51,9 @@ def _view(ptr: int, shape: tuple, dtype: torch.dtype, device) -> torch.Tensor:
     class _Mem:
         __cuda_array_interface__ = {"shape": (n,), "typestr": typestr, "data": (ptr, False), "version": 3}
 
-    t = torch.as_tensor(_Mem(), device=device)
+    mem = _Mem()
+    mem.owner = owner          # the tensor's storage holds `mem`
+    t = torch.as_tensor(mem, device=device)
     return (t.view(torch.bfloat16) if dtype == torch.bfloat16 else t).view(shape)
 
 
@@ -55,6 +69,7 @@ class MoeWorkspace:
                                          experts, topk, cap_rows, C.byref(self.h))
         if st != K.OK:
             raise XcclError(st, "xccl_moe_ws_create")
+        self._ws = _Workspace(self.h)
         self.tp = oob.size if oob is not None else emu_ranks
         self.n_local = 1 if oob is not None else emu_ranks
         self.cap_rows = int(K.load().xccl_moe_ws_cap_rows(self.h))
@@ -63,16 +78,16 @@ class MoeWorkspace:
         return int(K.load().xccl_moe_ws_buffer(self.h, local, which))
 
     def recv(self, local: int = 0) -> torch.Tensor:
-        return _view(self._buf(local, BUF_RECV), (self.cap_rows, self.H), torch.bfloat16, self.device)
+        return _view(self._buf(local, BUF_RECV), (self.cap_rows, self.H), torch.bfloat16, self.device, self._ws)
 
     def expert_out(self, local: int = 0) -> torch.Tensor:
-        return _view(self._buf(local, BUF_EXPERT_OUT), (self.cap_rows, self.H), torch.bfloat16, self.device)
+        return _view(self._buf(local, BUF_EXPERT_OUT), (self.cap_rows, self.H), torch.bfloat16, self.device, self._ws)
 
     def expert_rows(self, local: int = 0) -> torch.Tensor:
-        return _view(self._buf(local, BUF_EXPERT_ROWS), (self.E // self.tp + 1,), torch.int32, self.device)
+        return _view(self._buf(local, BUF_EXPERT_ROWS), (self.E // self.tp + 1,), torch.int32, self.device, self._ws)
 
     def row_source(self, local: int = 0) -> torch.Tensor:
-        return _view(self._buf(local, BUF_ROW_SOURCE), (self.cap_rows,), torch.int32, self.device)
+        return _view(self._buf(local, BUF_ROW_SOURCE), (self.cap_rows,), torch.int32, self.device, self._ws)
 
     def dispatch(self, x: Sequence[torch.Tensor], ids: Sequence[torch.Tensor]) -> None:
         st = K.load().xccl_moe_dispatch(self.h, _ptrs(x), _ptrs(ids), torch.cuda.current_stream().cuda_stream)
@@ -90,6 +105,6 @@ class MoeWorkspace:
         return int(K.load().xccl_moe_ws_error(self.h))
 
     def close(self) -> None:
-        if self.h:
-            K.load().xccl_moe_ws_destroy(self.h)
-            self.h = C.c_void_p()
+        """Gives the workspace up; its memory is freed now, or with the last tensor that views it."""
+        self.h = C.c_void_p()
+        self._ws = None
