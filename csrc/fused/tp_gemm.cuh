@@ -33,6 +33,7 @@ enum CommMode { COMM_NONE = 0, COMM_ALLGATHER_A = 1, COMM_REDUCE_SCATTER_C = 2 }
 
 struct GemmParams {
     int M, N, K;          // N counts accumulator columns (gate + up for SwiGLU)
+    int bn;               // bf16: accumulator columns of a tile (gemm_tile_cols; 0 = 256). The boxes of tmB0 / tmB1 are bn / 2 rows
     int epilogue;
     int comm;
     int tp_size;          // ranks taking part (1 without communication)
@@ -106,6 +107,9 @@ struct GemmLaunch {
 xccl_status_t make_tensor_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ld,
                                  uint32_t box_rows);
 
+// Columns of a bf16 tile for this product on `walkers` tile walkers (CTA pairs): 256, or less where that fills the last
+// wave of tiles better. A function of the sizes alone: every rank of a team gets the same answer.
+int gemm_tile_cols(int M, int N, int K, bool swiglu, int walkers);
 xccl_status_t launch_gemm(const GemmParams &p, const GemmLaunch &l, cudaStream_t stream);
 // The block-scaled fp8 kernel (tp_gemm_fp8.cu): same parameters; tmA / tmB0 / tmB1 are byte maps built by
 // make_tensor_map_u8 with boxes of 128 rows (A, plain B) or 64 rows (SwiGLU gate and up halves) x 128 bytes.

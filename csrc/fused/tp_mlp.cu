@@ -265,6 +265,7 @@ xccl_status_t xccl_tp_ag_gemm_swiglu(xccl_tp_ws_h w, const void *const *Wg, cons
     l.cooperative = w->tp > 1;
     p.n_gemm_ctas = ctas - copy_ctas;
     p.copy_mode   = w->copy_mode;
+    p.bn          = gemm_tile_cols(p.M, p.N, p.K, true, p.n_gemm_ctas / 2);
     for (int r = 0; r < w->tp; r++) {
         p.xg[r]  = w->xg(r);
         p.pad[r] = w->pad(r);
@@ -275,9 +276,9 @@ xccl_status_t xccl_tp_ag_gemm_swiglu(xccl_tp_ws_h w, const void *const *Wg, cons
         xccl_status_t st = make_tensor_map_2d(&l.tmA[i], w->xg(w->rank_base + i), (uint64_t)w->M, (uint64_t)w->K,
                                               (uint64_t)w->K, kBM);
         if (st != XCCL_OK) return st;
-        st = make_tensor_map_2d(&l.tmB0[i], Wg[i], (uint64_t)F_local, (uint64_t)w->K, (uint64_t)w->K, kBN / 2);
+        st = make_tensor_map_2d(&l.tmB0[i], Wg[i], (uint64_t)F_local, (uint64_t)w->K, (uint64_t)w->K, (uint32_t)p.bn / 2);
         if (st != XCCL_OK) return st;
-        st = make_tensor_map_2d(&l.tmB1[i], Wu[i], (uint64_t)F_local, (uint64_t)w->K, (uint64_t)w->K, kBN / 2);
+        st = make_tensor_map_2d(&l.tmB1[i], Wu[i], (uint64_t)F_local, (uint64_t)w->K, (uint64_t)w->K, (uint32_t)p.bn / 2);
         if (st != XCCL_OK) return st;
         if (w->in_active) p.in_ready[i] = w->in_flags[i];
     }
@@ -367,14 +368,15 @@ xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void
     p.seq       = ++w->seq_rs;
     p.error     = w->error;
     p.ldc       = w->N_rs;
-    const int tiles_n = (p.N + kBN - 1) / kBN;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    p.bn = gemm_tile_cols(p.M, p.N, p.K, false, sms / w->n_local / 2);
+    const int tiles_n = (p.N + p.bn - 1) / p.bn;
     w->rs_count[p.seq & 1] += (uint32_t)tiles_n;
     p.rs_target = w->rs_count[p.seq & 1];
     p.rs_fused  = w->rs_fused ? 1 : 0;
     p.rs_debug_local = w->rs_debug_local ? 1 : 0;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     l.n_local     = w->n_local;
     l.ctas        = sms / w->n_local;
     l.cooperative = w->emulated && w->tp > 1;  // emulated ranks wait on one another inside one launch
@@ -387,7 +389,7 @@ xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void
         p.C[i] = (__nv_bfloat16 *)Yout[i];
         xccl_status_t st = make_tensor_map_2d(&l.tmA[i], Hin[i], (uint64_t)w->M, (uint64_t)F_local, (uint64_t)F_local, kBM);
         if (st != XCCL_OK) return st;
-        st = make_tensor_map_2d(&l.tmB0[i], Wd[i], (uint64_t)w->N_rs, (uint64_t)F_local, (uint64_t)F_local, kBN / 2);
+        st = make_tensor_map_2d(&l.tmB0[i], Wd[i], (uint64_t)w->N_rs, (uint64_t)F_local, (uint64_t)F_local, (uint32_t)p.bn / 2);
         if (st != XCCL_OK) return st;
         l.tmB1[i] = l.tmB0[i];
     }
