@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../core/core.h"
@@ -57,30 +58,57 @@ namespace {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// One warp per (row, 128-column block): amax by shuffles, four values per lane.
-__global__ void __launch_bounds__(256) quantize_rows_1x128_kernel(const __nv_bfloat16 *x, int rows, int K, uint8_t *out,
-                                                                  float *scales)
+// Block of 128 columns b of the matrix (rows are contiguous and K is a multiple of 128, so blocks and their scales are
+// simply numbered through): amax by shuffles, one scale, e4m3 bytes. kV values per lane, 128 / kV lanes per block, eight
+// blocks per warp with their loads all in flight. What it costs is the traffic (3 bytes per value); with one block per
+// warp, 8-byte loads and nothing in flight beside them 4096 x 8192 (100 MB) took 43.8 us, now 20.3 us.
+// kV = 8 needs 16-byte aligned input and 8-byte aligned output, kV = 4 half of that.
+template <int kV> __global__ void __launch_bounds__(256) quantize_rows_1x128_kernel(const __nv_bfloat16 *x, size_t blocks,
+                                                                                  uint8_t *out, float *scales)
 {
-    const int    kb_per_row = K / 128;
-    const size_t warp  = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
-    const int    lane  = threadIdx.x % 32;
-    const size_t total = (size_t)rows * kb_per_row;
-    if (warp >= total) return;
-    const size_t row = warp / kb_per_row;
-    const int    kb  = (int)(warp % kb_per_row);
-    const uint2  raw = *reinterpret_cast<const uint2 *>(x + row * (size_t)K + (size_t)kb * 128 + lane * 4);
-    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw);
-    const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-    float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y)));
+    constexpr int kLanes = 128 / kV, kPer = 32 / kLanes, kU = 8 / kPer;  // lanes per block, blocks per warp at a time, times
+    const size_t  warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int     lane = threadIdx.x % 32, l = lane % kLanes;
+    const size_t  b0   = warp * 8 + lane / kLanes;
+    using Raw = typename std::conditional<kV == 8, uint4, uint2>::type;
+    Raw raw[kU];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float s = fmaxf(amax, 1e-12f) / 448.0f, inv = 1.0f / s;
-    uint32_t q = (uint32_t)__nv_cvt_float_to_fp8(a.x * inv, __NV_SATFINITE, __NV_E4M3) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(a.y * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(b.x * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(b.y * inv, __NV_SATFINITE, __NV_E4M3) << 24);
-    *reinterpret_cast<uint32_t *>(out + row * (size_t)K + (size_t)kb * 128 + lane * 4) = q;
-    if (lane == 0) scales[row * kb_per_row + kb] = s;
+    for (int u = 0; u < kU; u++) {
+        // (a warp past the end repeats the last block and stores nothing)
+        const size_t b = min(b0 + (size_t)u * kPer, blocks - 1);
+        raw[u] = __ldg(reinterpret_cast<const Raw *>(x + b * 128 + l * kV));
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+        const size_t          b = b0 + (size_t)u * kPer;
+        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[u]);
+        float2 v[kV / 2];
+        float  amax = 0.0f;
+#pragma unroll
+        for (int e = 0; e < kV / 2; e++) {
+            v[e] = __bfloat1622float2(h[e]);
+            amax = fmaxf(amax, fmaxf(fabsf(v[e].x), fabsf(v[e].y)));
+        }
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        const float s = fmaxf(amax, 1e-12f) / 448.0f, inv = 1.0f / s;
+        uint32_t q[kV / 4];
+#pragma unroll
+        for (int e = 0; e < kV / 4; e++) {
+            q[e] = (uint32_t)__nv_cvt_float_to_fp8(v[2 * e].x * inv, __NV_SATFINITE, __NV_E4M3) |
+                   ((uint32_t)__nv_cvt_float_to_fp8(v[2 * e].y * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
+                   ((uint32_t)__nv_cvt_float_to_fp8(v[2 * e + 1].x * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
+                   ((uint32_t)__nv_cvt_float_to_fp8(v[2 * e + 1].y * inv, __NV_SATFINITE, __NV_E4M3) << 24);
+        }
+        if (b < blocks) {
+            if (kV == 8) {
+                *reinterpret_cast<uint2 *>(out + b * 128 + l * kV) = make_uint2(q[0], q[kV / 4 - 1]);
+            } else {
+                *reinterpret_cast<uint32_t *>(out + b * 128 + l * kV) = q[0];
+            }
+            if (l == 0) scales[b] = s;
+        }
+    }
 }
 
 void layout(TpWorkspace *w)
@@ -402,10 +430,11 @@ xccl_status_t xccl_tp_quantize_rows(const void *x_bf16, int rows, int K, void *o
     if (x_bf16 == nullptr || out8 == nullptr || scales == nullptr || rows <= 0 || K <= 0 || K % 128 != 0) {
         return XCCL_ERR_INVALID_PARAM;
     }
-    const size_t warps  = (size_t)rows * (K / 128);
-    const size_t blocks = (warps * 32 + 255) / 256;
-    quantize_rows_1x128_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x_bf16, rows, K,
-                                                                                   (uint8_t *)out8, scales);
+    const size_t   blocks = (size_t)rows * (K / 128);
+    const unsigned grid   = (unsigned)((blocks + 63) / 64);   // eight warps of eight blocks
+    const bool     wide   = ((uintptr_t)x_bf16 & 15) == 0 && ((uintptr_t)out8 & 7) == 0;
+    auto           k      = wide ? quantize_rows_1x128_kernel<8> : quantize_rows_1x128_kernel<4>;
+    k<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x_bf16, blocks, (uint8_t *)out8, scales);
     XCCL_CUDA_CHECK(cudaGetLastError());
     return XCCL_OK;
 }

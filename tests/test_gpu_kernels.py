@@ -760,6 +760,23 @@ def test_quantize_rows_kernel_matches_torch(dev):
     _loaded_native()
 
 
+@pytest.mark.parametrize("rows,shift", [(1, 0), (1, 4), (9, 0), (63, 4), (64, 8), (65, 0)])
+def test_quantize_rows_edges_of_the_grid_and_alignments(dev, rows, shift):
+    """Block counts around a thread block's 64, an input that is only 8-byte aligned, and bytes behind the output."""
+    from xccl_b200.ops import gemm
+    from xccl_b200.ops.tp import quantize_rows
+    flat = (torch.randn(rows * 128 + 16, device=dev) * 3).to(torch.bfloat16)
+    x = flat[shift: shift + rows * 128].view(rows, 128)
+    out = torch.zeros(rows * 128 + 64, dtype=torch.uint8, device=dev)
+    s = torch.full((rows + 1,), -1.0, device=dev)
+    quantize_rows(x, out[: rows * 128].view(torch.float8_e4m3fn).view(rows, 128), s[:rows].view(rows, 1))
+    scale = x.float().abs().amax(-1, keepdim=True).clamp_min(1e-12) / gemm.FP8_MAX
+    torch.testing.assert_close(s[:rows, None], scale, rtol=1e-6, atol=0)
+    want = (x.float() * (1.0 / s[:rows, None])).to(torch.float8_e4m3fn)   # the same product, rounded once
+    assert torch.equal(out[: rows * 128].view(torch.float8_e4m3fn).view(rows, 128).float(), want.float())
+    assert float(s[rows]) == -1.0 and int(out[rows * 128:].sum()) == 0
+
+
 @pytest.mark.parametrize("tp,fuse_quant", [(1, True), (2, True), (4, True), (2, False)])
 def test_tp_mlp_fp8_fused_matches_dequantised_reference(dev, tp, fuse_quant):
     """fp8 allgather->GEMM+SwiGLU and GEMM->reduce-scatter (ranks emulated in one launch) against fp32
