@@ -439,6 +439,40 @@ def test_emu_collectives_under_the_bounds_checking_build(dev):
     assert "violations 0" in r.stdout
 
 
+@pytest.mark.parametrize("ranks,kb", [(2, 8192), (2, 16400), (4, 2048), (4, 4112), (4, 8208), (8, 1024), (8, 4096)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int32])
+def test_emu_large_collectives_with_no_algorithm_named(dev, ranks, kb, dtype):
+    """Around the sizes where the unnamed algorithm turns zero-copy, and the forms that must stay staged: types the
+    zero-copy kernels do not have, unaligned buffers. Integers, so sums are exact."""
+    from xccl_b200.ops.emu import EmuWorld
+    w = EmuWorld(ranks, 8 << 20)
+    try:
+        n = (kb << 10) // torch.empty(0, dtype=dtype).element_size() // (16 * ranks) * (16 * ranks)
+        pool = torch.randint(-8, 9, (ranks * (n + 16) + n,), device=dev).to(dtype)
+        for shift in (0, 1):                        # shift 1: sources that are not 16-byte aligned
+            src = [pool[r * (n + 16) + shift: r * (n + 16) + shift + n] for r in range(ranks)]
+            total = sum(s.double() for s in src)
+            dst = [torch.empty(n, dtype=dtype, device=dev) for _ in range(ranks)]
+            w.allreduce(src, dst)
+            assert all(torch.equal(d.double(), total) for d in dst)
+            part = [torch.empty(n // ranks, dtype=dtype, device=dev) for _ in range(ranks)]
+            w.reduce_scatter(src, part)
+            assert torch.equal(torch.cat(part).double(), total)
+            w.alltoall(src, dst)
+            chunks = [s.chunk(ranks) for s in src]
+            assert all(torch.equal(dst[d], torch.cat([chunks[s][d] for s in range(ranks)])) for d in range(ranks))
+            full = [torch.empty(n * ranks, dtype=dtype, device=dev) for _ in range(ranks)]
+            w.allgather(src, full)
+            assert all(torch.equal(f, torch.cat(src)) for f in full)
+        # in place
+        src = [pool[r * (n + 16): r * (n + 16) + n].clone() for r in range(ranks)]
+        total = sum(s.double() for s in src)
+        w.allreduce(src, src)
+        assert all(torch.equal(s.double(), total) for s in src)
+    finally:
+        w.close()
+
+
 def test_emu_sync_collectives_and_bounded_wait(world4, dev):
     for _ in range(3):
         world4.barrier()
