@@ -35,6 +35,7 @@ struct TpWorkspace {
     uint32_t *error = nullptr;
     size_t    off_xg = 0, off_part = 0, total = 0;
     uint32_t  seq_ag = 0, seq_rs = 0, rs_count[2] = {0, 0};
+    bool      copy_ctas_auto = true;
     int       copy_ctas = 0;      // CTAs of the allgather->GEMM kernel that pull the remote shards; 0 = by team size
     int       copy_mode = 1;      // 1: copier warps in every CTA, 0: whole copy CTAs
     bool      rs_debug_local = false;
@@ -111,6 +112,18 @@ template <int kV> __global__ void __launch_bounds__(256) quantize_rows_1x128_ker
     }
 }
 
+// CTAs per rank that pull the remote shards (copy mode 0). Emulated ranks share one GPU's SMs (37 CTAs per rank with four)
+// and copy inside its memory, and what the copy has to keep up with is the tile walk, whose time per byte of A grows with
+// the columns of B. Four ranks, 2048 x 4096 x 14336 (7168 columns per rank), block step with 10 / 6 / 4 / 2 copy CTAs: 689 /
+// 658 / 645 / 790 us, fp8 723 / 654 / 629 / 631; 1024 x 2048 x 4096 (2048 columns): 142 / 151 / 161 / 209.
+int copy_ctas_of(const TpWorkspace *w, int columns, int ctas)
+{
+    if (w->tp <= 1 || w->copy_mode != 0) return 0;
+    int want = w->copy_ctas;
+    if (w->emulated && w->copy_ctas_auto) want = std::min(want, std::max(2, (28672 + columns - 1) / columns));
+    return std::max(1, std::min(want, ctas / 4));
+}
+
 void layout(TpWorkspace *w)
 {
     w->off_xg   = align_up(nvl::kPadBytes, 4096);
@@ -185,6 +198,7 @@ xccl_status_t xccl_tp_ws_create(const xccl_oob_collectives_t *oob, int emu_ranks
     // Copy mode 1 (two copier warps in every CTA, plain loads) costs no tensor throughput but moves only about
     // 120 GB/s per GPU however many loads it keeps in flight (8 GPUs: 1.12 ms), enough for two ranks (67 MB in 2.5 ms:
     // 4.16 ms per block step against 4.41 ms with copy CTAs), not for eight.
+    w->copy_ctas_auto = w->copy_ctas <= 0;
     if (w->copy_ctas <= 0) w->copy_ctas = 16;
     if (w->copy_mode < 0) w->copy_mode = w->tp <= 2 ? 1 : 0;
     int tiles_m = (M + kBM - 1) / kBM;
@@ -287,7 +301,7 @@ xccl_status_t xccl_tp_ag_gemm_swiglu(xccl_tp_ws_h w, const void *const *Wg, cons
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int ctas      = sms / w->n_local;
-    int copy_ctas = (w->tp > 1 && w->copy_mode == 0) ? std::max(1, std::min(w->copy_ctas, ctas / 4)) : 0;
+    int copy_ctas = copy_ctas_of(w, p.N, ctas);
     l.n_local     = w->n_local;
     l.ctas        = ctas;
     l.cooperative = w->tp > 1;
@@ -492,7 +506,7 @@ xccl_status_t xccl_tp_ag_gemm_swiglu_fp8q(xccl_tp_ws_h w, const void *const *Wg8
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int ctas      = sms / w->n_local;
-    int copy_ctas = (w->tp > 1 && w->copy_mode == 0) ? std::max(1, std::min(w->copy_ctas, ctas / 4)) : 0;
+    int copy_ctas = copy_ctas_of(w, p.N, ctas);
     l.n_local     = w->n_local;
     l.ctas        = ctas;
     l.cooperative = w->tp > 1;
