@@ -94,16 +94,20 @@ __device__ __forceinline__ uint4 ld16_if(const void *p, bool on)
     return v;
 }
 
-// Go words of the offsets (ctl[0]); 0 between launches.
-constexpr uint32_t kGoRun = 1, kGoSkip = 2;
+// Go words of the offsets (ctl[0]); 0 between launches. kGoMeet: nothing is copied (a receive buffer is too small, or this
+// rank has failed before), but the ranks have met and meet again at the end. kGoSkip: they have not met.
+constexpr uint32_t kGoRun = 1, kGoSkip = 2, kGoMeet = 3;
 
 // Block 0 of each rank routes: it counts its entries per expert in shared memory (the atomic's return value is the
 // entry's position among its expert's), sends the E counts to every rank, and after one barrier every rank knows the
 // whole [tp][E] matrix and derives all offsets itself, so nobody reads a peer's offsets back. The other blocks wait for
-// its go word; the block that finishes last holds the closing barrier and clears the words for the next launch.
+// its go word; the block that finishes last holds the closing barrier and clears the words for the next launch. The
+// closing barrier follows every opening one that was met, rows or none: a rank that ran ahead into its next dispatch would
+// overwrite the counts a peer is still adding up, and the peer, one epoch behind, would take the wrong flags for its own.
+// Returns the go word.
 // The routing is a serial chain that every row waits for: with the offsets added up by one thread over E loads and
 // three grid-wide barriers around it, 128 tokens x 7168, 256 experts, top 8, took 102 us for a 5 us copy.
-__device__ bool route_block0(const MoeParams &p, int local, int rank)
+__device__ uint32_t route_block0(const MoeParams &p, int local, int rank)
 {
     __shared__ uint32_t s_cnt[kMaxExperts];
     __shared__ uint32_t s_warp[32];
@@ -189,7 +193,7 @@ __device__ bool route_block0(const MoeParams &p, int local, int rank)
     }
     __threadfence();
     __syncthreads();
-    return ok;
+    return !met ? kGoSkip : ok && *(volatile uint32_t *)p.error[local] == 0 ? kGoRun : kGoMeet;
 }
 
 __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams p)
@@ -201,10 +205,10 @@ __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams 
     __shared__ uint32_t s_go;
 
     if (blockIdx.x == 0) {
-        const bool ok = route_block0(p, local, rank);
+        const uint32_t go = route_block0(p, local, rank);
         if (threadIdx.x == 0) {
-            s_go = (ok && *(volatile uint32_t *)p.error[local] == 0) ? kGoRun : kGoSkip;
-            st_release_gpu(ctl, s_go);
+            s_go = go;
+            st_release_gpu(ctl, go);
         }
     } else if (threadIdx.x == 0) {
         const unsigned long long t0 = nvl::global_ns();
@@ -270,13 +274,16 @@ __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams 
     __threadfence_system();
     __syncthreads();
     __shared__ int s_last;
-    if (threadIdx.x == 0) s_last = atomicAdd(ctl + 1, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(ctl + 1, 1u) == gridDim.x - 1;
+        if (s_last != 0) s_go = *(volatile uint32_t *)ctl;   // block 0's word, also where this block gave up waiting for it
+    }
     __syncthreads();
     if (s_last == 0) return;
     // the last block of this rank: everything has landed everywhere before anyone returns
     __threadfence_system();
     if (threadIdx.x == 0) ctl[0] = ctl[1] = 0;
-    if (s_go == kGoRun && p.tp > 1) {
+    if (s_go != kGoSkip && p.tp > 1) {
         uint32_t epoch = *(volatile uint32_t *)(p.pad[rank] + nvl::kPadEpochOff);
         bool     ok    = cross_rank_barrier(p, rank, 0, epoch);
         if (threadIdx.x == 0) {
@@ -563,6 +570,16 @@ uint32_t xccl_moe_ws_error(xccl_moe_ws_h w)
         if (v != 0) worst = v;
     }
     return worst;
+}
+
+// Barriers that a local rank has held on flag row 0 (dispatch: two, also when it copies nothing; combine: two of its
+// block 0), for tests. Synchronises.
+uint32_t xccl_moe_ws_meetings(xccl_moe_ws_h w, int local_rank)
+{
+    uint32_t v = 0;
+    if (w == nullptr || local_rank < 0 || local_rank >= w->p.n_local) return 0xffffffffu;
+    cudaMemcpy(&v, w->p.pad[w->p.rank_base + local_rank] + nvl::kPadEpochOff, 4, cudaMemcpyDeviceToHost);
+    return v;
 }
 
 }  // extern "C"

@@ -37,6 +37,7 @@ xccl_status_t xccl_moe_combine(xccl_moe_ws_h ws, const int32_t *const *ids, cons
 void         *xccl_moe_ws_buffer(xccl_moe_ws_h ws, int local_rank, int which);
 int           xccl_moe_ws_cap_rows(xccl_moe_ws_h ws);
 uint32_t      xccl_moe_ws_error(xccl_moe_ws_h ws);  // 0 = fine; synchronises
+uint32_t      xccl_moe_ws_meetings(xccl_moe_ws_h ws, int local_rank);  // barriers held with the peers (tests); synchronises
 
 #ifdef __cplusplus
 }

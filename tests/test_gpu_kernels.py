@@ -679,6 +679,45 @@ def test_moe_dispatch_combine_matches_reference(dev, ranks):
         ws.close()
 
 
+@pytest.mark.parametrize("ranks", [1, 2, 4])
+def test_moe_receive_buffer_too_small(dev, ranks):
+    """One rank's receive buffer is a row too small: every rank reports it, nobody writes a row, and the ranks meet at the
+    end of every dispatch all the same, so that none runs ahead into its next one (rows or not: two barriers each)."""
+    import ctypes as C
+    from xccl_b200.ops.moe import MoeWorkspace
+    T, H, E, Kk = 40, 64, 8, 2
+    ws = MoeWorkspace(T, H, E, Kk, emu_ranks=ranks, cap_rows=ranks * T * Kk - 1)
+    fn = K.load().xccl_moe_ws_meetings
+    fn.restype, fn.argtypes = C.c_uint32, [C.c_void_p, C.c_int]
+    meetings = lambda: [fn(ws.h, r) for r in range(ranks)]
+    per = 2 if ranks > 1 else 0                       # one rank has nobody to meet
+    try:
+        xs = [torch.randn(T, H, device=dev).to(torch.bfloat16) for _ in range(ranks)]
+        spread = [torch.randint(0, E, (T, Kk), dtype=torch.int32, device=dev) for _ in range(ranks)]
+        fits = [(s + torch.arange(T, device=dev)[:, None]).remainder(E).to(torch.int32) for s in spread]
+        full = [torch.zeros(T, Kk, dtype=torch.int32, device=dev) for _ in range(ranks)]   # all rows to expert 0
+        if ranks > 1:
+            ws.dispatch(xs, fits)
+            assert ws.error() == 0 and meetings() == [per] * ranks
+        else:
+            per = 0
+        for r in range(ranks):
+            ws.recv(r).fill_(7.0)
+            ws.row_source(r).fill_(-9)
+        base = meetings()
+        for it in range(1, 4):
+            ws.dispatch(xs, full)
+            assert all(bool((ws.recv(r) == 7.0).all()) and bool((ws.row_source(r) == -9).all()) for r in range(ranks))
+            assert ws.error() == 0x400
+            assert meetings() == [b + it * per for b in base]
+        outs = [torch.full((T, H), 3.0, dtype=torch.bfloat16, device=dev) for _ in range(ranks)]
+        ws.combine(full, [torch.ones(T, Kk, device=dev) for _ in range(ranks)], outs)
+        assert ws.error() == 0x400 and all(bool((o == 3.0).all()) for o in outs)
+        assert meetings() == [b + 4 * per for b in base]
+    finally:
+        ws.close()
+
+
 def test_moe_views_outlive_the_workspace(dev):
     """A tensor on workspace memory keeps that memory after close(); without views close() frees it."""
     from xccl_b200.ops.moe import MoeWorkspace
