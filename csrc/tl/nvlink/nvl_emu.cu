@@ -188,14 +188,16 @@ xccl_status_t xccl_nvlink_emu_collective(void *world, int coll_type, const void 
     cfg.blocks      = blocks;
     cudaStream_t  s = (cudaStream_t)stream;
     xccl_status_t st;
-    // emulated ranks share one address space: the "registered" peer buffers are the buffers themselves
+    // emulated ranks share one address space: the "registered" peer buffers are the buffers themselves (in the zero-copy
+    // call alone: a staged kernel has no business in a peer's buffer, and the bounds-checking build holds it to that)
+    Call direct = c;
     for (int r = 0; r < w.size; r++) {
-        c.peer_src[r] = c.src[r];
-        c.peer_dst[r] = c.dst[r];
+        direct.peer_src[r] = c.src[r];
+        direct.peer_dst[r] = c.dst[r];
     }
-    if (alg == ALG_AUTO && direct_pays(w, c, coll_type, (xccl_dt_t)dt, (xccl_dt_t)out_dt)) alg = ALG_DIRECT;
+    if (alg == ALG_AUTO && direct_pays(w, direct, coll_type, (xccl_dt_t)dt, (xccl_dt_t)out_dt)) alg = ALG_DIRECT;
     if (alg == ALG_DIRECT) {
-        st = launch_direct(w, c, coll_type, (xccl_dt_t)dt, (xccl_dt_t)out_dt, cfg, s);
+        st = launch_direct(w, direct, coll_type, (xccl_dt_t)dt, (xccl_dt_t)out_dt, cfg, s);
         if (st != XCCL_OK) return st;
         XCCL_CUDA_CHECK(cudaStreamSynchronize(s));
         for (int r = 0; r < w.size; r++) {

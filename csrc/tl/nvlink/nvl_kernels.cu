@@ -883,6 +883,7 @@ __global__ void timeout_probe_kernel(World w, unsigned long long budget_ns)
 #ifdef XCCL_DEBUG_BOUNDS
 // Ranges a launch may touch with its 16-byte accesses: every rank's workspace, the multicast mapping, and what the call
 // names (registered peer buffers, symmetric buffers through the multicast mapping) with generous but finite extents.
+DbgRanges g_dbg_last{};  // those of the last launch, for xccl_nvlink_debug_bounds_ranges
 void dbg_set_ranges(const World &w, const Call &c, cudaStream_t stream)
 {
     DbgRanges r{};
@@ -901,6 +902,7 @@ void dbg_set_ranges(const World &w, const Call &c, cudaStream_t stream)
     }
     add(c.mc_src[0], span);
     add(c.mc_dst[0], span);
+    g_dbg_last = r;
     cudaMemcpyToSymbolAsync(g_dbg, &r, sizeof(r), 0, cudaMemcpyHostToDevice, stream);
 }
 template <typename... R> void dbg_prepare(cudaStream_t s, World w, Call c, R...) { dbg_set_ranges(w, c, s); }
@@ -1198,6 +1200,23 @@ xccl_status_t launch_timeout_probe(const World &w, unsigned long long budget_ns,
 
 }  // namespace nvl
 }  // namespace xccl
+
+// Ranges that the last launch was entitled to in the bounds-checking build: lo[i], hi[i] of up to `max`; returns their
+// number, or -1 in a library built without XCCL_DEBUG_BOUNDS.
+extern "C" int xccl_nvlink_debug_bounds_ranges(unsigned long long *lo, unsigned long long *hi, int max)
+{
+#ifdef XCCL_DEBUG_BOUNDS
+    const auto &r = xccl::nvl::g_dbg_last;
+    for (int i = 0; i < r.n && i < max; i++) {
+        lo[i] = (unsigned long long)(uintptr_t)r.lo[i];
+        hi[i] = (unsigned long long)(uintptr_t)r.hi[i];
+    }
+    return r.n;
+#else
+    (void)lo; (void)hi; (void)max;
+    return -1;
+#endif
+}
 
 // Record of the bounds-checking build: out[0] = accesses that were refused since the last call, out[1] = the first
 // refused address, out[2] = its kind (1 store, 2 load, 3 multicast store, 4 multicast load), out[3] = (rank << 32) |

@@ -439,6 +439,47 @@ def test_emu_collectives_under_the_bounds_checking_build(dev):
     assert "violations 0" in r.stdout
 
 
+_RANGES_SCRIPT = r"""
+import ctypes as C, torch
+from xccl_b200 import _capi as K
+from xccl_b200.ops.emu import EmuWorld
+dev = torch.device("cuda:0")
+lo, hi = (C.c_ulonglong * 64)(), (C.c_ulonglong * 64)()
+n, ws = 2, 1 << 20
+w = EmuWorld(n, ws)
+def may_touch(t):
+    k = K.load().xccl_nvlink_debug_bounds_ranges(lo, hi, 64)
+    assert 0 < k <= 64
+    a, b = t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()
+    return any(lo[i] < b and a < hi[i] for i in range(k))
+big = 16 << 20                        # 16 MB and more of all ranks together run zero-copy when no algorithm is named
+for count, alg, direct in ((1024, 0, False), (1024, K.NVLINK_ALG_TWO_SHOT, False), (big // 8, K.NVLINK_ALG_TWO_SHOT, False),
+                           (big // 8, 0, True), (1024, K.NVLINK_ALG_DIRECT, True)):
+    src = [torch.ones(count, device=dev) for _ in range(n)]
+    dst = [torch.empty(count, device=dev) for _ in range(n)]
+    w.allreduce(src, dst, alg=alg)
+    assert all(bool((d == n).all()) for d in dst)
+    assert [may_touch(t) for t in src + dst] == [direct] * 2 * n, (count, alg)
+w.close()
+print("ranges ok")
+"""
+
+
+def test_bounds_of_a_staged_collective_leave_the_user_buffers_out(dev):
+    """The bounds-checking build entitles a staged kernel's checked accesses to the workspaces alone; the ranks' buffers
+    are added for the zero-copy kernels only."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parent.parent
+    lib = root / "xccl_b200" / "lib" / "libxccl_bounds.so"
+    if not lib.exists():
+        pytest.skip("libxccl_bounds.so is not built (python -m xccl_b200.build --debug-bounds)")
+    env = dict(os.environ, XCCL_B200_LIB=str(lib), PYTHONPATH=str(root))
+    r = subprocess.run([sys.executable, "-c", _RANGES_SCRIPT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
 @pytest.mark.parametrize("ranks,kb", [(2, 8192), (2, 16400), (4, 2048), (4, 4112), (4, 8208), (8, 1024), (8, 4096)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int32])
 def test_emu_large_collectives_with_no_algorithm_named(dev, ranks, kb, dtype):
