@@ -107,9 +107,19 @@ struct GemmLaunch {
 xccl_status_t make_tensor_map_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ld,
                                  uint32_t box_rows);
 
-// Columns of a bf16 tile for this product on `walkers` tile walkers (CTA pairs): 256, or less where that fills the last
-// wave of tiles better. A function of the sizes alone: every rank of a team gets the same answer.
-int gemm_tile_cols(int M, int N, int K, bool swiglu, int walkers);
+// How launch_gemm lays a product out: CTA pairs on 256-row tiles or single CTAs on 128-row tiles, and how many of them
+// walk the tiles of a rank. `may_pair`: the option and the device allow pairs.
+struct TileWalk {
+    bool pair;
+    int  walkers;
+};
+TileWalk tile_walk(int M, int tp_size, CommMode comm, int ctas, int n_gemm_ctas, int copy_mode, bool may_pair);
+// The same for a launch that is being prepared (p.M, tp_size, comm, n_gemm_ctas and copy_mode are set) on the current device.
+TileWalk tile_walk(const GemmParams &p, const GemmLaunch &l);
+
+// Columns of a bf16 tile for this product: 256, or less where that fills the last wave of tiles better. It depends on the
+// sizes and on the device's SM count; the ranks of a team need not agree on it.
+int gemm_tile_cols(int M, int N, int K, bool swiglu, const TileWalk &walk);
 xccl_status_t launch_gemm(const GemmParams &p, const GemmLaunch &l, cudaStream_t stream);
 // The block-scaled fp8 kernel (tp_gemm_fp8.cu): same parameters; tmA / tmB0 / tmB1 are byte maps built by
 // make_tensor_map_u8 with boxes of 128 rows (A, plain B) or 64 rows (SwiGLU gate and up halves) x 128 bytes.

@@ -307,7 +307,7 @@ xccl_status_t xccl_tp_ag_gemm_swiglu(xccl_tp_ws_h w, const void *const *Wg, cons
     l.cooperative = w->tp > 1;
     p.n_gemm_ctas = ctas - copy_ctas;
     p.copy_mode   = w->copy_mode;
-    p.bn          = gemm_tile_cols(p.M, p.N, p.K, true, p.n_gemm_ctas / 2);
+    p.bn          = gemm_tile_cols(p.M, p.N, p.K, true, tile_walk(p, l));
     for (int r = 0; r < w->tp; r++) {
         p.xg[r]  = w->xg(r);
         p.pad[r] = w->pad(r);
@@ -413,16 +413,16 @@ xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    p.bn = gemm_tile_cols(p.M, p.N, p.K, false, sms / w->n_local / 2);
+    l.n_local     = w->n_local;
+    l.ctas        = sms / w->n_local;
+    p.n_gemm_ctas = l.ctas;
+    p.bn          = gemm_tile_cols(p.M, p.N, p.K, false, tile_walk(p, l));
     const int tiles_n = (p.N + p.bn - 1) / p.bn;
     w->rs_count[p.seq & 1] += (uint32_t)tiles_n;
     p.rs_target = w->rs_count[p.seq & 1];
     p.rs_fused  = w->rs_fused ? 1 : 0;
     p.rs_debug_local = w->rs_debug_local ? 1 : 0;
-    l.n_local     = w->n_local;
-    l.ctas        = sms / w->n_local;
     l.cooperative = w->emulated && w->tp > 1;  // emulated ranks wait on one another inside one launch
-    p.n_gemm_ctas = l.ctas;
     for (int r = 0; r < w->tp; r++) {
         p.part[r] = w->part(r);
         p.pad[r]  = w->pad(r);

@@ -1,0 +1,44 @@
+"""How the tensor-parallel GEMM lays a launch out (``csrc/fused/tp_gemm.cu``), asked on the CPU: pairs or single CTAs, how
+many of them walk tiles, and the tile width that is chosen for exactly these walkers."""
+import pytest
+
+from xccl_b200 import _capi as K
+
+NONE, ALLGATHER, REDUCE_SCATTER = 0, 1, 2
+
+
+def _walk(M, tp, comm, ctas, gemm, copy_mode=0, may_pair=1):
+    v = K.load().xccl_tp_tile_walk(M, tp, comm, ctas, gemm, copy_mode, may_pair)
+    return v < 0, abs(v)
+
+
+def _cost(M, N, bn, walkers):
+    tiles = -(-M // 256) * (-(-N // bn))
+    return -(-tiles // walkers) * (bn + 110)
+
+
+@pytest.mark.parametrize("ctas", [2, 3, 18, 37, 49, 74, 148])
+def test_walkers_are_those_of_the_launch(ctas):
+    for copy in range(0, ctas // 4 + 1):
+        pair, walkers = _walk(4096, 4, ALLGATHER, ctas, ctas - copy)
+        # the grid has an even number of CTAs, the copiers take an even number of them
+        want = (ctas - ctas % 2 - (copy + copy % 2)) // 2
+        if want >= 1:
+            assert (pair, walkers) == (True, want)
+        assert _walk(4096, 4, ALLGATHER, ctas, ctas - copy, may_pair=0) == (False, ctas - copy)
+        assert _walk(4096, 4, ALLGATHER, ctas, ctas - copy, copy_mode=1)[1] == ctas // 2     # the copiers are warps
+    # shards of 384 rows are no whole 256-row tiles; without communication any row count is
+    assert _walk(1536, 4, REDUCE_SCATTER, ctas, ctas) == (False, ctas)
+    assert _walk(1536, 4, NONE, ctas, ctas) == (True, ctas // 2)
+
+
+def test_width_is_chosen_for_the_walkers_of_the_launch():
+    """Four ranks of 37 CTAs with nine that copy: the odd one copies too and 13 pairs walk, not 14. 28 tiles of 160 columns
+    would be two waves of 14 but are three of 13."""
+    M, N, k = 1024, 1024, 3072
+    pair, walkers = _walk(M, 4, ALLGATHER, 37, 37 - 9)
+    assert (pair, walkers) == (True, 13)
+    bn = K.load().xccl_tp_tile_cols(M, N, k, 1, int(pair), walkers)
+    assert _cost(M, N, bn, walkers) == min(_cost(M, N, b, walkers) for b in range(64, 257, 32)) and bn == 192
+    # single CTAs keep 256 columns
+    assert K.load().xccl_tp_tile_cols(M, N, k, 1, 0, walkers) == 256
