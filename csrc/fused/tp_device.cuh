@@ -513,7 +513,7 @@ __device__ void rs_reduce_phase(const GemmParams &p, int rank, int local, int ti
         if (threadIdx.x == 0) {
             int good = 1;
             for (int src = 0; src < p.tp_size && good; src++) {
-                // rs_target = tiles that rank `src` has sent for this row block over all launches
+                // rs_target = what the tiles that rank `src` sends for this row block have added over all launches
                 // of this parity, this one included (the host keeps the running total)
                 good = wait_counter(ctr_base + src * 64 + mb_in, p.rs_target, true, ab, 6) ? 1 : 0;
             }

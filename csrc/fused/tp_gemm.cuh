@@ -59,7 +59,7 @@ struct GemmParams {
     int       sync_kblocks;               // 0 = only at tile starts
     unsigned  sync_budget_ns;
     uint32_t seq;         // launch sequence number (starts at 1): readiness counters and buffer parity follow it
-    uint32_t rs_target;   // reduce-scatter: running total of tiles per (source, row block) for this parity
+    uint32_t rs_target;   // reduce-scatter: running total of arrivals (rs_arrivals) per (source, row block) for this parity
     int      rs_debug_local;  // diagnostic (wrong results): partial tiles go to local memory and nobody is waited for
     int      rs_fused;    // reduce-scatter: 1 = the tiles of the local rows (walked last) add the other ranks' partial
                           // tiles in their epilogue and write the result; 0 = a reduce phase after the last tile
@@ -116,6 +116,16 @@ struct TileWalk {
 TileWalk tile_walk(int M, int tp_size, CommMode comm, int ctas, int n_gemm_ctas, int copy_mode, bool may_pair);
 // The same for a launch that is being prepared (p.M, tp_size, comm, n_gemm_ctas and copy_mode are set) on the current device.
 TileWalk tile_walk(const GemmParams &p, const GemmLaunch &l);
+
+// What a finished partial tile `nb` of `bn` columns adds to its owner's arrival counter: the 32-column pieces it holds of
+// the N output columns. All tiles of a row block come to rs_arrivals_total(N) whatever their width, so the ranks of a team
+// need not cut their tiles alike (bn is a multiple of 32; it follows the SM count of the rank's device).
+__host__ __device__ constexpr uint32_t rs_arrivals_total(int N) { return (uint32_t)((N + 31) / 32); }
+__host__ __device__ constexpr uint32_t rs_arrivals(int N, int bn, int nb)
+{
+    const int lo = nb * bn, hi = lo + bn < N ? lo + bn : N;
+    return (uint32_t)((hi - lo + 31) / 32);
+}
 
 // Columns of a bf16 tile for this product: 256, or less where that fills the last wave of tiles better. It depends on the
 // sizes and on the device's SM count; the ranks of a team need not agree on it.

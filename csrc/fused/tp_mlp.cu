@@ -417,8 +417,7 @@ xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void
     l.ctas        = sms / w->n_local;
     p.n_gemm_ctas = l.ctas;
     p.bn          = gemm_tile_cols(p.M, p.N, p.K, false, tile_walk(p, l));
-    const int tiles_n = (p.N + p.bn - 1) / p.bn;
-    w->rs_count[p.seq & 1] += (uint32_t)tiles_n;
+    w->rs_count[p.seq & 1] += rs_arrivals_total(p.N);
     p.rs_target = w->rs_count[p.seq & 1];
     p.rs_fused  = w->rs_fused ? 1 : 0;
     p.rs_debug_local = w->rs_debug_local ? 1 : 0;
@@ -561,7 +560,7 @@ xccl_status_t xccl_tp_gemm_rs_fp8(xccl_tp_ws_h w, const void *const *H8, const f
     p.seq       = ++w->seq_rs;
     p.error     = w->error;
     p.ldc       = w->N_rs;
-    w->rs_count[p.seq & 1] += (uint32_t)((p.N + kBN - 1) / kBN);  // tiles per row block
+    w->rs_count[p.seq & 1] += rs_arrivals_total(p.N);
     p.rs_target = w->rs_count[p.seq & 1];
     p.rs_fused  = w->rs_fused ? 1 : 0;
     p.rs_debug_local = w->rs_debug_local ? 1 : 0;

@@ -42,3 +42,13 @@ def test_width_is_chosen_for_the_walkers_of_the_launch():
     assert _cost(M, N, bn, walkers) == min(_cost(M, N, b, walkers) for b in range(64, 257, 32)) and bn == 192
     # single CTAs keep 256 columns
     assert K.load().xccl_tp_tile_cols(M, N, k, 1, 0, walkers) == 256
+
+
+@pytest.mark.parametrize("N", [8, 32, 40, 256, 264, 1000, 4096, 8200])
+def test_arrivals_of_a_row_block_do_not_depend_on_the_tile_width(N):
+    """The owner of a row block waits for a count that a rank on another device, with other tiles, reaches as well."""
+    fn = K.load().xccl_tp_rs_arrivals
+    total = fn(N, 0, -1)
+    for bn in range(32, 257, 32):
+        parts = [fn(N, bn, nb) for nb in range(-(-N // bn))]
+        assert all(p > 0 for p in parts) and sum(parts) == total
