@@ -18,6 +18,7 @@
 //              up the tokens it owns over the cluster (distributed shared memory, in rank order: same bits every run),
 //              applies the epilogue and writes rows of 128 outputs
 #include <algorithm>
+#include <atomic>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -411,6 +412,66 @@ SkinnyKernel skinny_kernel_of(int mn, bool fp8, bool swiglu)
     }
 }
 
+int kernel_index(int mn, bool fp8, bool swiglu)
+{
+    return !fp8 ? (swiglu ? 1 : 0) : 2 + 2 * (mn == 32 ? 0 : mn == 64 ? 1 : 2) + (swiglu ? 1 : 0);
+}
+
+// Dynamic shared memory of a CTA when `occ` of them share an SM (228 KB, 1 KB of it taken by each CTA).
+constexpr int skinny_smem_budget(int occ) { return (occ == 2 ? 113 : 226) * 1024 - 64; }
+
+// The largest number of CTAs up to `splits` (halved where it does not fit) that the device places as one cluster.
+template <typename F> int placeable(int splits, F &&fits)
+{
+    while (splits > 1 && !fits(splits)) splits = (splits + 1) / 2;
+    return splits;
+}
+
+void launch_config(const SkinnyPlan &plan, bool fp8, cudaStream_t stream, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr)
+{
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim          = dim3((unsigned)plan.splits, (unsigned)plan.tiles);
+    cfg->blockDim         = dim3(fp8 ? kSkinnyThreadsFp8 : kSkinnyThreads);
+    cfg->dynamicSmemBytes = (size_t)plan.smem_bytes;
+    cfg->stream           = stream;
+    attr->id               = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)plan.splits;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg->attrs    = attr;
+    cfg->numAttrs = 1;
+}
+
+// Sets the kernel up on this device and lowers plan->splits to a cluster that it places: a partitioned device may have no
+// room for eight CTAs in one GPC. Asked once per device, kernel and cluster size (properties that do not change, and the
+// kernel's largest shared memory stands for all of its plans).
+xccl_status_t prepare_kernel(SkinnyKernel k, int dev, bool fp8, bool swiglu, SkinnyPlan *plan)
+{
+    static std::atomic<unsigned char> ready[64][8], fit[64][8][9];   // fit: 0 not asked, 1 yes, 2 no
+    const int id = kernel_index(plan->mn, fp8, swiglu);
+    if (ready[dev][id].load() == 0) {
+        XCCL_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        ready[dev][id].store(1);
+    }
+    plan->splits = placeable(plan->splits, [&](int s) {
+        auto &f = fit[dev][id][s];
+        if (f.load() == 0) {
+            SkinnyPlan         q = *plan;
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr[1];
+            q.splits     = s;
+            q.smem_bytes = skinny_smem_budget(skinny_occupancy(plan->mn, fp8, swiglu));
+            launch_config(q, fp8, nullptr, &cfg, attr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) (void)cudaGetLastError();
+            if (clusters < 1) xccl_warn("few-rows gemm: no room for a cluster of %d CTAs on device %d", s, dev);
+            f.store(clusters >= 1 ? 1 : 2);
+        }
+        return f.load() == 1;
+    });
+    return XCCL_OK;
+}
+
 }  // namespace
 
 bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
@@ -425,8 +486,7 @@ bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan
     const int occ     = skinny_occupancy(q.mn, fp8, swiglu);
     const int stage   = (int)kWBytes * mats + q.mn * 128;
     const int fixed   = 1024 + (int)kBarBytes + (fp8 ? kScaleSlots * mats * q.mn * 4 : 0);
-    // shared memory of an SM: 228 KB, 1 KB of it taken by each CTA
-    const int budget  = (occ == 2 ? 113 : 226) * 1024 - 64;
+    const int budget  = skinny_smem_budget(occ);
     q.stages  = std::min(kMaxStages, (budget - fixed) / stage);
     q.cols    = mats * (fp8 ? q.mn : (q.mn + 31) / 32 * 32);
     q.nbuf    = fp8 ? std::max(1, std::min(kMaxBuf, 512 / occ / q.cols)) : 1;
@@ -451,7 +511,9 @@ bool try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st)
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
     if (!skinny_plan(a.M, a.N, a.K, a.fp8, a.swiglu, sms, &plan)) return false;
     *st = launch_skinny(a, plan, stream);
-    return true;
+    if (*st == XCCL_OK) return true;
+    (void)cudaGetLastError();   // refused: the large kernel serves the call, or says why not
+    return false;
 }
 
 xccl_status_t launch_skinny(const SkinnyArgs &a, const SkinnyPlan &plan, cudaStream_t stream)
@@ -477,32 +539,24 @@ xccl_status_t launch_skinny(const SkinnyArgs &a, const SkinnyPlan &plan, cudaStr
     if ((st = map(&maps.b0, a.B0, a.N, 128)) != XCCL_OK) return st;
     if ((st = map(&maps.b1, a.swiglu ? a.B1 : a.B0, a.N, 128)) != XCCL_OK) return st;
     SkinnyKernel k = skinny_kernel_of(plan.mn, a.fp8, a.swiglu);
-    static bool  attr_set[64][8] = {};
     int          dev = 0;
     XCCL_CUDA_CHECK(cudaGetDevice(&dev));
-    const int id = !a.fp8 ? (a.swiglu ? 1 : 0) : 2 + 2 * (plan.mn == 32 ? 0 : plan.mn == 64 ? 1 : 2) + (a.swiglu ? 1 : 0);
-    if (!attr_set[dev][id]) {
-        XCCL_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        attr_set[dev][id] = true;
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3((unsigned)plan.splits, (unsigned)plan.tiles);
-    cfg.blockDim         = dim3(a.fp8 ? kSkinnyThreadsFp8 : kSkinnyThreads);
-    cfg.dynamicSmemBytes = (size_t)plan.smem_bytes;
-    cfg.stream           = stream;
+    if ((st = prepare_kernel(k, dev, a.fp8, a.swiglu, &p.plan)) != XCCL_OK) return st;
+    cudaLaunchConfig_t  cfg;
     cudaLaunchAttribute attr[1];
-    attr[0].id               = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)plan.splits;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs    = attr;
-    cfg.numAttrs = 1;
+    launch_config(p.plan, a.fp8, stream, &cfg, attr);
     XCCL_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k, p, maps));
     return XCCL_OK;
 }
 
 }  // namespace tp
 }  // namespace xccl
+
+// Host-side view of the cluster that is launched (tests): `splits` CTAs are wanted, bit s of `fits` says that s are placed.
+extern "C" int xccl_tp_skinny_cluster(int splits, unsigned fits)
+{
+    return xccl::tp::placeable(splits, [&](int s) { return (fits >> s & 1u) != 0; });
+}
 
 // Host-side view of the cut (tests): out = {mn, tiles, splits, kblocks, stages, nbuf, cols, tmem_cols, chunk, smem_bytes,
 // CTAs per SM}. Returns 1 when the sizes are served by this kernel, 0 otherwise.

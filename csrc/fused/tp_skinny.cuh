@@ -36,7 +36,8 @@ struct SkinnyPlan {
 };
 // False when the sizes are not for this kernel (the callers then use launch_gemm / launch_gemm_fp8).
 bool          skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *plan);
-// Runs the product here when its sizes are for this kernel: true, with the launch's status in *st.
+// Runs the product here when its sizes are for this kernel and the device takes the launch (true); otherwise nothing has
+// been launched and the caller's large kernel serves it.
 bool          try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st);
 xccl_status_t launch_skinny(const SkinnyArgs &a, const SkinnyPlan &plan, cudaStream_t stream);
 

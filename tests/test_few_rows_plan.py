@@ -43,3 +43,16 @@ def test_plan_covers_the_product_and_fits_the_sm(fp8, swiglu):
 def test_more_rows_than_one_mma_are_left_to_the_large_kernel():
     assert _plan(129, 8192, 8192, False, False) is None
     assert _plan(0, 8192, 8192, False, False) is None
+
+
+def test_a_cluster_the_device_does_not_place_becomes_a_smaller_one():
+    """A partitioned device may place no cluster of eight: the call is served with fewer CTAs per tile instead of refused.
+    One CTA always fits."""
+    fn = K.load().xccl_tp_skinny_cluster
+    for splits in range(1, 9):
+        assert fn(splits, 0x1ff) == splits
+        assert fn(splits, 0) == 1
+        for most in range(1, 9):
+            got = fn(splits, (2 << most) - 1)
+            assert 1 <= got <= min(splits, most)
+            assert got == splits or got >= min(splits, most) / 2
