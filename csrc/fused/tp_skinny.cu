@@ -4,11 +4,14 @@
 // or 128 rows its grid is N / 256 CTA pairs that each walk all of K: 32 of 74 pairs for N = 8192, and half of the SMs'
 // loads are never issued. Here the operands change places: 128 rows of the WEIGHTS are the M side of tcgen05.mma, the
 // activations (rounded up to 16 rows) its N side, and the CTAs of a cluster share the K blocks of a tile, so that the
-// grid fills the chip with about two CTAs per SM and each keeps its whole ring of weight loads in flight.
-// Measured on one B200, operands in DRAM, before (large kernel) and now: bf16 16 x 8192 x 8192 (134 MB of weights)
-// 47.5 -> 26.5 us, 128 x 8192 x 8192 49.0 -> 34.2 us, 128 x 2048 x 8192 46.1 -> 22.2 us; SwiGLU 16 x 3584 x 8192
-// 69.0 -> 26.2 us; fp8 64 x 7168 x 8192 49.2 -> 18.6 us. At 128 rows the smallest K (128 x 8192 x 256) is equal at 10.3 us,
-// so the line lies at the 128 rows that one MMA holds, for every N and K.
+// grid fills the chip (up to two CTAs per SM, one in fp8 with more than 32 tokens or SwiGLU) and each keeps its whole ring
+// of weight loads in flight. Measured on one B200, operands in DRAM, before (large kernel with 256-column tiles) and now: bf16
+// 16 x 8192 x 8192 (134 MB of weights) 47.5 -> 26.5 us, 128 x 8192 x 8192 49.0 -> 34.2 us; SwiGLU 16 x 3584 x 8192 69.0 ->
+// 26.2 us; fp8 64 x 7168 x 8192 49.2 -> 18.6 us.
+// The line lies at the 128 rows that one MMA holds. On both sides of it at 128 rows, this kernel / the large one with the
+// narrower tiles it now has, L2 flushed, event times in steps of 2 us: bf16 N 8192, K 8192 40.9 / 53.2, K 2048 20.5 / 20.7,
+// K 512 15.7 / 14.6; N 2048, K 1024 16.3 / 14.5 (K up to 1024 is where the large one is level or up to 2 us ahead); SwiGLU N
+// 8192, K 2048 37 / 50; fp8 N 8192, K 2048 19 / 26, N 28672, K 512 22.3 / 20.6.
 //
 //   warp 0     TMA producer: weights (streamed, evict first) and activations (kept in L2) of a K block per stage
 //   warp 1     MMA issuer, accumulators in tensor memory: lane = weight row, column = token
@@ -474,6 +477,38 @@ xccl_status_t prepare_kernel(SkinnyKernel k, int dev, bool fp8, bool swiglu, Ski
 
 }  // namespace
 
+namespace {
+
+// CTAs that share the K blocks of a tile: as many as run in one wave, as long as each gets enough K blocks to be worth its
+// launch and its part of the reduction. A cluster lies inside one GPC: a B200 with room for 296 of these CTAs (148 with one
+// per SM) places 71 (33) clusters of four, 45 (22) of six and 33 (15) of eight, so clusters may take 7/8 of the room, those
+// of eight 3/4; pairs always fit. How many K blocks are enough depends on who else is there: four while half of the SMs are
+// free, eight while every CTA has an SM to itself (16 for the large clusters, whose reduction is longer), 32 where two share
+// an SM and one more only splits its bandwidth; for pairs always four.
+// us with 1 / 2 / 3 / 4 / 6 / 8 CTAs per tile, L2 flushed, event times in steps of 2 us, the large kernel last:
+//   bf16  16 x 1024 x  8192   32.8 / 22.5 / 18.4 / 18.0 / 16.4 / 14.4   39.1
+//   bf16 128 x 4096 x  2048   24.6 / 19.8 / 18.4 / 18.4 / 22.5 / 24.7   18.6
+//   bf16 128 x 6144 x  2048   24.6 / 20.4 / 21.5 / 22.6 / 32.8 / 36.9   20.6
+//   bf16 128 x 6144 x 28672    178 /  106 / 90.1 / 80.3 /  107 / 99.4    123
+//   bf16 128 x 8192 x  8192   61.5 / 43.0 / 41.0 / 40.9 / 57.3 / 59.1   53.2
+//   fp8   64 x 2048 x  8192   26.7 / 20.5 / 18.5 / 18.5 / 18.5 / 26.7   43.2
+//   fp8  128 x 5120 x 28672    115 / 65.7 / 51.2 / 78.3 / 67.6 / 82.5    133
+int skinny_share(int tiles, int kblocks, int occ, int sms)
+{
+    int best = 1;
+    for (int s : {2, 3, 4, 6, 8}) {
+        const int ctas = s * tiles, room = occ * sms;
+        if (ctas > (s == 2 ? room : s == 8 ? room * 3 / 4 : room * 7 / 8)) continue;
+        int least = 32;
+        if (ctas <= sms / 2 || s == 2) least = 4;
+        else if (ctas <= sms) least = s >= 6 ? 16 : 8;
+        if (kblocks >= least * s) best = s;
+    }
+    return best;
+}
+
+}  // namespace
+
 bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
 {
     if (M <= 0 || M > kSkinnyMaxM || N <= 0 || K <= 0) return false;
@@ -491,10 +526,7 @@ bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan
     q.cols    = mats * (fp8 ? q.mn : (q.mn + 31) / 32 * 32);
     q.nbuf    = fp8 ? std::max(1, std::min(kMaxBuf, 512 / occ / q.cols)) : 1;
     q.tmem_cols = pow2_at_least(q.nbuf * q.cols, 32);
-    // K is shared out until the CTAs of one wave fill the chip; at least four K blocks each, so that a CTA's ring of
-    // loads is worth its launch and its part of the reduction. 16 x 1024 x 8192 with 8 / 4 / 2 / 1 CTAs per tile: 10.5 /
-    // 13.8 / 18.2 / 29.6 us; 128 x 8192 x 8192 with 4 / 2 / 1: 34.2 / 35.0 / 53.7 us
-    q.splits  = std::max(1, std::min(std::min(8, occ * sms / q.tiles), q.kblocks / 4));
+    q.splits  = skinny_share(q.tiles, q.kblocks, occ, sms);
     q.chunk   = std::min(q.mn, q.stages * stage / (512 * mats) / 16 * 16);
     q.smem_bytes = fixed + q.stages * stage;
     if (q.stages < 2 || q.chunk < 16) return false;

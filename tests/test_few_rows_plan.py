@@ -56,3 +56,26 @@ def test_a_cluster_the_device_does_not_place_becomes_a_smaller_one():
             got = fn(splits, (2 << most) - 1)
             assert 1 <= got <= min(splits, most)
             assert got == splits or got >= min(splits, most) / 2
+
+
+# clusters of 1 .. 8 CTAs that a B200 holds at a time, with one and with two CTAs per SM
+B200 = {1: (0, 148, 74, 45, 33, 26, 22, 15, 15), 2: (0, 296, 148, 93, 71, 56, 45, 37, 33)}
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_tiles_run_in_one_wave_of_the_clusters_a_gpu_holds(fp8, swiglu):
+    """K is shared only while all tiles' clusters are resident at once: a second wave costs more than a longer K loop."""
+    for M in (1, 16, 33, 64, 100, 128):
+        for N in range(128, 40001, 128):
+            for K_ in (128, 512, 2048, 8192, 28672):
+                p = _plan(M, N, K_, fp8, swiglu)
+                assert p["splits"] == 1 or (p["tiles"] <= B200[p["occ"]][p["splits"]] and p["kblocks"] >= 4 * p["splits"])
+
+
+@pytest.mark.parametrize("M,N,K_,fp8,swiglu,splits", [
+    (16, 8192, 8192, False, False, 4), (128, 8192, 28672, False, False, 4), (64, 7168, 8192, True, False, 2),
+    (128, 6144, 2048, False, False, 3), (128, 6144, 4096, False, True, 3), (128, 4096, 2048, False, False, 4),
+    (64, 2048, 8192, True, False, 4), (16, 1024, 8192, False, False, 8), (128, 28672, 8192, False, True, 1)])
+def test_share_at_the_measured_sizes(M, N, K_, fp8, swiglu, splits):
+    assert _plan(M, N, K_, fp8, swiglu)["splits"] == splits
