@@ -98,7 +98,9 @@ namespace {
 // staged / zero-copy in us, by the bytes of all ranks together: allreduce fp32 8 ranks 2 MB 30.7 / 34.2, 8 MB 47.3 /
 // 34.3, 128 MB 151.5 / 83.2, 2 ranks 8 MB 30.2 / 36.6, 16 MB (bf16) 45.4 / 34.5; reduce-scatter 8 ranks 8 MB 30.6 / 31.6, 32 MB
 // 46.9 / 39.6, 128 MB 104 / 59.5; allgather (output) 8 ranks 64 MB 45.5 / 52.4, 256 MB 120.9 / 105.6; alltoall 8 ranks 16 MB 35.4 /
-// 42.3, 32 MB 48.8 / 44.9, 128 MB 135.2 / 82.8.
+// 42.3, 128 MB 135.2 / 82.8. Around the limits: reduce-scatter fp32 4 ranks 20 MB 32.3 / 37.1, 28 MB 37.3 / 38.3, 36
+// MB 42.8 / 39.2, 8 ranks 20 MB 36.3 / 35.2, bf16 4 ranks 16 MB 35.3 / 31.8; allgather 4 ranks 100 MB 60.8 / 61.1, 128 MB 76.4 / 70.1, 6 ranks 112 MB 58.2 / 61.6, 8 ranks 144 MB 64.9 / 74.6, 192 MB
+// 95.2 / 87.7; alltoall 4 ranks 32 MB 46.6 / 47.8, 8 ranks 36 MB 45.9 / 49.6, 40 MB 53.2 / 55.0, 48 MB 67.1 / 59.0.
 bool direct_pays(const World &w, const Call &c, int coll, xccl_dt_t dt, xccl_dt_t out_dt)
 {
     if (out_dt == XCCL_DT_UNSUPPORTED || out_dt == XCCL_DT_LAST_PREDEFINED) out_dt = dt;
@@ -117,16 +119,16 @@ bool direct_pays(const World &w, const Call &c, int coll, xccl_dt_t dt, xccl_dt_
         if (!typed) return false;
         src_bytes = c.count * es * n;
         dst_bytes = c.count * xccl_dt_size(out_dt);
-        least     = (size_t)16 << 20;
+        least     = (size_t)(es >= 4 && n < 8 ? 32 : 16) << 20;
         break;
     case XCCL_ALLGATHER:
         src_bytes = c.len / n;
         dst_bytes = c.len;
-        least     = (size_t)100 << 20;
+        least     = (size_t)(n >= 8 ? 160 : n >= 6 ? 120 : 100) << 20;
         break;
     case XCCL_ALLTOALL:
         src_bytes = dst_bytes = c.len * n;
-        least     = (size_t)32 << 20;
+        least     = (size_t)(n >= 8 ? 48 : 32) << 20;
         break;
     default: return false;
     }
@@ -250,6 +252,22 @@ xccl_status_t xccl_nvlink_emu_collective(void *world, int coll_type, const void 
         if (e->status(r).code != NVL_OK) return XCCL_ERR_NO_MESSAGE;
     }
     return XCCL_OK;
+}
+
+// Whether a collective on these buffers runs zero-copy when no algorithm is named (tests; the buffers are not touched).
+int xccl_nvlink_emu_direct_pays(int nranks, int coll_type, const void *const *srcs, void *const *dsts, size_t count, size_t len,
+                                int dt, int out_dt)
+{
+    World w{};
+    Call  c{};
+    w.size = nranks;
+    for (int r = 0; r < nranks; r++) {
+        c.src[r] = c.peer_src[r] = srcs[r];
+        c.dst[r] = c.peer_dst[r] = dsts[r];
+    }
+    c.count = count;
+    c.len   = len;
+    return direct_pays(w, c, coll_type, (xccl_dt_t)dt, (xccl_dt_t)out_dt) ? 1 : 0;
 }
 
 xccl_status_t xccl_nvlink_emu_timeout_probe(void *world, int budget_ms, float *elapsed_ms, uint32_t *status4)
