@@ -112,16 +112,22 @@ template <int kV> __global__ void __launch_bounds__(256) quantize_rows_1x128_ker
     }
 }
 
-// CTAs per rank that pull the remote shards (copy mode 0). Emulated ranks share one GPU's SMs (37 CTAs per rank with four)
-// and copy inside its memory, and what the copy has to keep up with is the tile walk, whose time per byte of A grows with
-// the columns of B. Four ranks, 2048 x 4096 x 14336 (7168 columns per rank), block step with 10 / 6 / 4 / 2 copy CTAs: 689 /
-// 658 / 645 / 790 us, fp8 723 / 654 / 629 / 631; 1024 x 2048 x 4096 (2048 columns): 142 / 151 / 161 / 209.
+// CTAs per rank that pull the remote shards (copy mode 0): `want`, or with `emulated_auto` fewer where that pays. Emulated
+// ranks share one GPU's SMs (37 CTAs per rank with four) and copy inside its memory, and what the copy has to keep up with is
+// the tile walk, whose time per byte of A grows with the columns of B. Four ranks, 2048 x 4096 x 14336 (7168 columns per
+// rank), block step with 10 / 6 / 4 / 2 copy CTAs: 689 / 658 / 645 / 790 us, fp8 723 / 654 / 629 / 631; 1024 x 2048 x 4096 (2048
+// columns): 142 / 151 / 161 / 209. Shards of a single 128-row block want the shard sooner than the walk of one block covers:
+// three ranks, 384 x 4096 x 14208, 12 / 6 / 4 copy CTAs 243 / 257 / 260 us, fp8 190 / 202 / 204; there all copy that may.
+// (3, 4 and 8 ranks, 134 sizes, against 16 everywhere: 1 to 2 % less with 256 rows and more per shard, up to 11 %.)
+int copy_ctas(int tp, int copy_mode, int want, bool emulated_auto, int shard_rows, int columns, int ctas)
+{
+    if (tp <= 1 || copy_mode != 0) return 0;
+    if (emulated_auto && shard_rows >= 2 * kBM) want = std::min(want, std::max(2, (28672 + columns - 1) / columns));
+    return std::max(1, std::min(want, ctas / 4));
+}
 int copy_ctas_of(const TpWorkspace *w, int columns, int ctas)
 {
-    if (w->tp <= 1 || w->copy_mode != 0) return 0;
-    int want = w->copy_ctas;
-    if (w->emulated && w->copy_ctas_auto) want = std::min(want, std::max(2, (28672 + columns - 1) / columns));
-    return std::max(1, std::min(want, ctas / 4));
+    return copy_ctas(w->tp, w->copy_mode, w->copy_ctas, w->emulated && w->copy_ctas_auto, w->M / w->tp, columns, ctas);
 }
 
 void layout(TpWorkspace *w)
@@ -385,6 +391,12 @@ xccl_status_t xccl_tp_h2d_begin(xccl_tp_ws_h w, const void *const *host_x, void 
 {
     xccl_status_t st = xccl_tp_h2d_expect(w, copy_stream, 1);
     return st != XCCL_OK ? st : xccl_tp_h2d_issue(w, host_x, copy_stream);
+}
+
+// Host-side view of the number of copy CTAs (tests).
+int xccl_tp_copy_ctas(int tp, int copy_mode, int want, int emulated_auto, int shard_rows, int columns, int ctas)
+{
+    return copy_ctas(tp, copy_mode, want, emulated_auto != 0, shard_rows, columns, ctas);
 }
 
 xccl_status_t xccl_tp_gemm_rs(xccl_tp_ws_h w, const void *const *Hin, const void *const *Wd, void *const *Yout,

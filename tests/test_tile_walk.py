@@ -52,3 +52,15 @@ def test_arrivals_of_a_row_block_do_not_depend_on_the_tile_width(N):
     for bn in range(32, 257, 32):
         parts = [fn(N, bn, nb) for nb in range(-(-N // bn))]
         assert all(p > 0 for p in parts) and sum(parts) == total
+
+
+@pytest.mark.parametrize("tp", [3, 4, 8])
+def test_copy_ctas_of_emulated_ranks(tp):
+    """Fewer copy CTAs for wide products, but not where a shard is one 128-row block: its rows are wanted at once."""
+    fn, ctas = K.load().xccl_tp_copy_ctas, 148 // tp
+    most = min(16, ctas // 4)
+    for columns in (512, 2048, 7168, 28672):
+        assert fn(tp, 0, 16, 1, 128, columns, ctas) == most
+        assert fn(tp, 0, 16, 0, 1024, columns, ctas) == most            # real ranks, or a number that was asked for
+        assert fn(tp, 0, 16, 1, 256, columns, ctas) == max(1, min(most, max(2, -(-28672 // columns))))
+        assert fn(tp, 1, 16, 1, 256, columns, ctas) == 0 and fn(1, 0, 16, 1, 256, columns, 148) == 0
