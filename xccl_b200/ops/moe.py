@@ -31,13 +31,16 @@ def _ptrs(ts: Sequence[torch.Tensor]):
 
 
 class _Workspace:
-    """The native workspace; its memory is freed with the last reference to it."""
+    """The native workspace; its memory is freed with the last reference to it. One that is still referenced when the
+    interpreter ends goes with the process."""
 
     def __init__(self, h: C.c_void_p):
         self.h = h
 
     def __del__(self):
-        K.load().xccl_moe_ws_destroy(self.h)
+        load = getattr(K, "load", None)      # the module may be gone by then
+        if load is not None:
+            load().xccl_moe_ws_destroy(self.h)
 
 
 def _view(ptr: int, shape: tuple, dtype: torch.dtype, device, owner: _Workspace) -> torch.Tensor:
@@ -105,6 +108,7 @@ class MoeWorkspace:
         return int(K.load().xccl_moe_ws_error(self.h))
 
     def close(self) -> None:
-        """Gives the workspace up; its memory is freed now, or with the last tensor that views it."""
+        """Gives the workspace up; its memory is freed now, or with the last tensor that views it. Freeing waits for the
+        device, so neither this nor the end of the last view may fall into a graph capture."""
         self.h = C.c_void_p()
         self._ws = None
