@@ -720,6 +720,62 @@ def test_moe_dispatch_combine_matches_reference(dev, ranks):
         ws.close()
 
 
+@pytest.mark.parametrize("ranks,T,H,E,Kk", [
+    (1, 96, 8, 16, 1), (2, 64, 264, 16, 4),          # a row of one pack; a second, ragged piece of one pack
+    (1, 50, 1032, 64, 9), (2, 30, 520, 64, 33),      # more than eight entries per token in combine, more than 32 in dispatch
+    (4, 20, 7168, 16, 4), (1, 300, 2048, 1024, 8),   # 28 pieces of a row; as many experts as there are
+    (1, 6400, 1032, 16, 2), (1, 9500, 1032, 16, 2),  # pieces of 64 and of 128 packs (two and four loads per lane), ragged
+])
+def test_moe_row_pieces_many_entries_and_dropped_ids(dev, ranks, T, H, E, Kk):
+    """Sizes at which dispatch and combine cut rows and entries differently, with ids outside the experts among them."""
+    from xccl_b200.ops.moe import MoeWorkspace
+    EL = E // ranks
+    ws = MoeWorkspace(T, H, E, Kk, emu_ranks=ranks)
+    try:
+        g = torch.Generator(device=dev).manual_seed(T + H)
+        xs = [torch.randn(T, H, device=dev, generator=g).to(torch.bfloat16) for _ in range(ranks)]
+        ids = [torch.rand(T, E, device=dev, generator=g).topk(Kk, -1).indices.to(torch.int32) for _ in range(ranks)]
+        for i in ids:                                 # dropped entries, a whole token among them
+            drop = torch.rand(T, Kk, device=dev, generator=g) < 0.1
+            i[drop] = -1
+            i[T // 2] = E
+        gates = [torch.rand(T, Kk, device=dev, generator=g) for _ in range(ranks)]
+        x_all, ids_all = torch.stack(xs), torch.stack(ids).long()
+        ws.dispatch(xs, ids)
+        assert ws.error() == 0
+        for r in range(ranks):
+            rows = ws.expert_rows(r).long()
+            n = int(rows[EL])
+            want = torch.stack([(ids_all == e).sum() for e in range(r * EL, (r + 1) * EL)])
+            assert torch.equal(rows[:EL], want) and n == int(want.sum())
+            src = ws.row_source(r)[:n].long()
+            e = torch.repeat_interleave(torch.arange(r * EL, (r + 1) * EL, device=dev), rows[:EL])
+            assert torch.equal(ws.recv(r)[:n], x_all[src // T, src % T])
+            # every (expert, source, token) that was asked for exactly once, sources in order inside an expert
+            s_, t_, k_ = torch.nonzero((ids_all >= r * EL) & (ids_all < (r + 1) * EL), as_tuple=True)
+            asked = (ids_all[s_, t_, k_] * ranks + s_) * T + t_
+            assert torch.equal(((e * ranks + src // T) * T + src % T).sort().values, asked.sort().values)
+            key = e * ranks + src // T
+            assert bool((key[1:] >= key[:-1]).all())
+            ws.expert_out(r)[:n] = (ws.recv(r)[:n].float() * (1.0 + (e % 7)[:, None])).to(torch.bfloat16)
+        outs = [torch.full((T, H), 5.0, dtype=torch.bfloat16, device=dev) for _ in range(ranks)]
+        ws.combine(ids, gates, outs)
+        assert ws.error() == 0
+        for r in range(ranks):
+            want, size = torch.zeros(T, H, device=dev), torch.zeros(T, H, device=dev)
+            for k in range(Kk):
+                valid = ((ids[r][:, k] >= 0) & (ids[r][:, k] < E)).float()[:, None]
+                y = (xs[r].float() * (1.0 + (ids[r][:, k] % 7).float()[:, None])).to(torch.bfloat16).float()
+                want += valid * gates[r][:, k:k + 1] * y
+                size += valid * gates[r][:, k:k + 1] * y.abs()
+            # for every eight entries one bf16 rounding (half of its spacing: 2^-8) of a sum no larger than `size` and the
+            # roundings before it (3 %); fp32 sums beside it
+            assert bool(((outs[r].float() - want).abs() <= (-(-Kk // 8) * 1.03 * 2.0 ** -8 + 1e-5) * size).all())
+            assert not bool(outs[r][T // 2].any())    # a token without experts
+    finally:
+        ws.close()
+
+
 @pytest.mark.parametrize("ranks", [1, 2, 4])
 def test_moe_receive_buffer_too_small(dev, ranks):
     """One rank's receive buffer is a row too small: every rank reports it, nobody writes a row, and the ranks meet at the
@@ -854,6 +910,55 @@ def test_tp_mlp_one_block_of_rows_matches_reference(dev, fp8):
         assert float((got - want).abs().max()) <= tol * float(want.abs().max()) + 1e-3
     finally:
         mlp.close()
+
+
+_TILE_SCRIPT = r"""
+import torch
+from xccl_b200.ops import gemm
+from xccl_b200.models.tp_mlp import TpMlp, reference_forward_fp32
+dev = torch.device("cuda:0")
+g = torch.Generator(device=dev).manual_seed(1)
+R = lambda *s, scale=1.0: (torch.randn(*s, device=dev, generator=g) * scale).to(torch.bfloat16)
+for M, N, K in ((129, 8, 64), (257, 264, 136), (400, 1000, 520), (640, 232, 4104)):
+    a, b = R(M, K), R(N, K)
+    out = torch.full((M + 2, N), 7.0, device=dev, dtype=torch.bfloat16)
+    gemm.gemm_bf16(a, b, out[1:M + 1])
+    # bf16 rounding of the result (2^-8 of it) and fp32 sums of K products of size 1
+    torch.testing.assert_close(out[1:M + 1].float(), a.float() @ b.float().t(), rtol=1e-2, atol=1e-2 * K ** 0.5)
+    assert bool((out[0] == 7).all()) and bool((out[M + 1] == 7).all())
+for M, F, K in ((129, 128, 64), (300, 384, 1000)):
+    a, wg, wu = R(M, K), R(F, K, scale=K ** -0.5), R(F, K, scale=K ** -0.5)
+    out = torch.full((M + 2, F), 7.0, device=dev, dtype=torch.bfloat16)
+    gemm.gemm_swiglu(a, wg, wu, out[1:M + 1])
+    want = torch.nn.functional.silu(a.float() @ wg.float().t()) * (a.float() @ wu.float().t())
+    torch.testing.assert_close(out[1:M + 1].float(), want, rtol=1e-2, atol=1e-2)
+    assert bool((out[0] == 7).all()) and bool((out[M + 1] == 7).all())
+assert gemm.last_error() == 0
+for tokens, tp in ((512, 2), (768, 2), (384, 3)):      # shards of whole 256-row tiles and of single 128-row blocks
+    mlp = TpMlp(tokens, 264, 384 * tp, tp=tp)
+    x = R(tokens, 264)
+    for _ in range(2):
+        y = torch.cat(mlp.forward(list(x.chunk(tp, 0))), 0).float()
+        mlp.check_error()
+    want = reference_forward_fp32(x, torch.cat(mlp.w_gate, 0), torch.cat(mlp.w_up, 0), torch.cat(mlp.w_down, 1))
+    # two bf16 roundings and one of every rank's partial sum
+    assert float((y - want).abs().max()) <= 0.02 * float(want.abs().max()) + 1e-3, (tokens, tp)
+    mlp.close()
+print("tiles ok")
+"""
+
+
+@pytest.mark.parametrize("cols,pair", [(32, "y"), (32, "n"), (64, "n"), (160, "y"), (224, "y"), (224, "n")])
+def test_gemm_tiles_of_every_kind_of_width(dev, cols, pair):
+    """Tiles of a width that is asked for, as CTA pairs and as single CTAs (whose second half of B follows the first at
+    half a tile), over ragged rows and columns and through the allgather and reduce-scatter forms. The options are read
+    once per process."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    env = dict(os.environ, PYTHONPATH=str(Path(__file__).resolve().parent.parent), XCCL_TP_GEMM_BN=str(cols), XCCL_TP_GEMM_PAIR=pair)
+    r = subprocess.run([sys.executable, "-c", _TILE_SCRIPT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "tiles ok" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
 
 
 def test_quantize_rows_kernel_matches_torch(dev):
