@@ -40,8 +40,22 @@ def test_width_is_chosen_for_the_walkers_of_the_launch():
     assert (pair, walkers) == (True, 13)
     bn = K.load().xccl_tp_tile_cols(M, N, k, 1, int(pair), walkers)
     assert _cost(M, N, bn, walkers) == min(_cost(M, N, b, walkers) for b in range(64, 257, 32)) and bn == 192
-    # single CTAs keep 256 columns
-    assert K.load().xccl_tp_tile_cols(M, N, k, 1, 0, walkers) == 256
+
+
+@pytest.mark.parametrize("M,N,k,swiglu,walkers,cols", [
+    (512, 1280, 1280, 0, 37, 160),       # reduce-scatter, four ranks: 20 tiles on 37 walkers, 32 of 160 columns
+    (512, 8192, 1280, 0, 37, 256),       # 128 tiles, four waves whatever the width
+    (512, 5120, 1280, 1, 28, 256),       # three waves of 80 tiles; narrower ones promise 12 %, too little with SwiGLU
+    (256, 512, 1024, 1, 74, 64),         # four tiles, or sixteen
+    (2048, 512, 4096, 0, 148, 64)])
+def test_width_of_single_cta_tiles(M, N, k, swiglu, walkers, cols):
+    """128-row tiles: the least (waves x (columns + 370)), taken if it saves 10 % (20 % with SwiGLU)."""
+    def cost(b):
+        tiles = -(-M // 128) * (-(-(N // 2) // (b // 2)) if swiglu else -(-N // b))
+        return -(-tiles // walkers) * (b + 370)
+    got = K.load().xccl_tp_tile_cols(M, N, k, swiglu, 0, walkers)
+    least = min(range(64, 257, 32), key=lambda b: (cost(b), -b))
+    assert got == (least if cost(least) <= (0.8 if swiglu else 0.9) * cost(256) else 256) == cols
 
 
 @pytest.mark.parametrize("N", [8, 32, 40, 256, 264, 1000, 4096, 8200])
