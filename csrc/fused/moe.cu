@@ -115,6 +115,7 @@ __device__ uint32_t route_block0(const MoeParams &p, int local, int rank)
     const int      EL = p.E / p.tp, nent = p.T * p.K;
     const int32_t *ids = p.ids[local];
     const int      lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+    const uint32_t failed = *(volatile uint32_t *)p.error[local];   // by an earlier launch; asked here, where nobody waits for it
     for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) s_cnt[e] = 0;
     __syncthreads();
     // eight entries per thread in flight: the ids are the only memory latency of the count
@@ -193,7 +194,7 @@ __device__ uint32_t route_block0(const MoeParams &p, int local, int rank)
     }
     __threadfence();
     __syncthreads();
-    return !met ? kGoSkip : ok && *(volatile uint32_t *)p.error[local] == 0 ? kGoRun : kGoMeet;
+    return !met ? kGoSkip : ok && failed == 0 ? kGoRun : kGoMeet;
 }
 
 __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams p)
@@ -276,7 +277,8 @@ __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams 
     __shared__ int s_last;
     if (threadIdx.x == 0) {
         s_last = atomicAdd(ctl + 1, 1u) == gridDim.x - 1;
-        if (s_last != 0) s_go = *(volatile uint32_t *)ctl;   // block 0's word, also where this block gave up waiting for it
+        // block 0's word, also where this block gave up waiting for it (one rank alone has no barrier to decide on)
+        if (s_last != 0 && p.tp > 1) s_go = *(volatile uint32_t *)ctl;
     }
     __syncthreads();
     if (s_last == 0) return;
