@@ -27,6 +27,15 @@ constexpr uint32_t kSmemBytes  = kStages * kStageBytes + kEpiBytes + 256 + 1024;
 constexpr int      kStagesPair = 6;
 static_assert(kStagesPair * (kABytes + kBBytes / 2) == kStages * kStageBytes, "both modes share one shared-memory layout");
 
+// fp8: registers of a thread of the first four warps (loads, MMAs, copiers) and of the eight promotion warps, whose 128 running
+// sums spill with the 168 that twelve warps get alike.
+// fp8: products of the two scales of K blocks ahead, [slot][weight block][row].
+constexpr int      kScaleRing = 4;
+constexpr uint32_t kScaleRingBytes = 2 * kBM * 4;
+// fp8: registers of a thread of the first four warps (loads, MMAs, copier, scales) and of the eight promotion warps, whose 128
+// running sums and 32 values on their way spill with the 168 that twelve warps get alike.
+constexpr int      kRegsOthers = 104, kRegsPromotion = 200;
+
 struct Tile {
     int mb, nb, shard;
 };
@@ -358,10 +367,10 @@ __device__ void copy_cta_loop(const GemmParams &p, int rank, int local, int copy
 // issues them, so the copy is spread over all SMs, where it needs about 1.5 GB/s from each and costs no tensor
 // throughput. CTA 0's copiers also run the two cross-rank barriers (peers have published their shards / everybody
 // has finished reading) and release the other CTAs through a counter in local memory.
-constexpr int kCopierThreads = 64;
 constexpr int kGoSlot = 1100, kDoneSlot = 1101;  // words of the pad's counter area (the reduce-scatter counters end at 1024)
 
-template <int kU>   // 16-byte loads a thread keeps in flight (as many as the kernel's register budget allows)
+// kU: 16-byte loads a thread keeps in flight; the fp8 kernel has one warp of 32 threads for it, the bf16 kernel two.
+template <int kU, int kCopierThreads>
 __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int tid, const AbortFlag &ab)
 {
     const int    n_cta   = gridDim.x;
@@ -379,7 +388,10 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
     const size_t slo  = min((size_t)me * sper, sblk_packs), shi = min(slo + sper, sblk_packs);
     uint32_t    *go   = p.pad[rank] + nvl::kPadCounterOff + kGoSlot;
     uint32_t    *done = p.pad[rank] + nvl::kPadCounterOff + kDoneSlot;
-    auto sync_copiers = [] { asm volatile("bar.sync 6, 64;" ::: "memory"); };
+    auto sync_copiers = [] {
+        if (kCopierThreads == 32) __syncwarp();
+        else asm volatile("bar.sync 6, %0;" ::"n"(kCopierThreads) : "memory");
+    };
     bool ok = true;
 
     if (me == 0) {

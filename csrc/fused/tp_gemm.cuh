@@ -25,7 +25,7 @@ namespace tp {
 
 constexpr int kBM = 128, kBN = 256, kBK = 64, kStages = 4;
 constexpr int kThreads = 256;           // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue, warps 6-7: copiers (allgather mode)
-constexpr int kThreadsFp8 = 384;        // block-scaled fp8: warps 2-9 promote the per-K-block products and run the epilogue, 10-11 copy
+constexpr int kThreadsFp8 = 384;        // block-scaled fp8: warp 2 copies, 3 multiplies scales, 4-11 promote the per-K-block products and run the epilogue
 constexpr int kMaxTpRanks = 8;
 
 enum Epilogue { EPI_STORE = 0, EPI_SWIGLU = 1 };

@@ -849,6 +849,25 @@ def test_gemm_fp8_blockscaled_matches_dequantised_reference(dev, M, N, K_):
     torch.testing.assert_close(out.float(), want, rtol=2e-2, atol=2e-2 * float(want.abs().max()))
 
 
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("M,N,K_", [(129, 128, 128), (130, 384, 256), (255, 256, 384), (513, 640, 512), (257, 128, 640), (300, 896, 1152)])
+def test_gemm_fp8_blockscaled_scale_groups(dev, M, N, K_, off):
+    """Scales reach the kernel four K blocks at a time, 16 bytes per row where the rows are aligned: numbers of K blocks
+    around the groups, scales that do not start on 16 bytes, a last tile half outside N."""
+    from xccl_b200.ops import gemm
+    a = torch.randn(M, K_, device=dev) * torch.rand(M, 1, device=dev) * 3
+    b = torch.randn(N, K_, device=dev) * 0.05 * torch.rand(N // 128, device=dev).repeat_interleave(128)[:, None]
+    a8, sa = gemm.quantize_act_1x128(a)
+    b8, sb = gemm.quantize_weight_128x128(b)
+    moved = torch.full((sa.numel() + 8,), float("nan"), device=dev)[off:off + sa.numel()].view_as(sa)
+    moved.copy_(sa)
+    out = gemm.gemm_fp8_blockscaled(a8, moved, b8, sb)
+    assert gemm.last_error() == 0
+    want = gemm.dequantize(a8, sa, 1).double() @ gemm.dequantize(b8, sb, 128).double().t()
+    # half a unit in the last place of bf16 (2^-9), and 32-bit sums of K products far below the largest value
+    torch.testing.assert_close(out.double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+
+
 @pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 127, 128, 129])
 @pytest.mark.parametrize("N,K_", [(8, 8), (264, 520), (1024, 4104)])
 def test_gemm_few_rows_matches_fp32_reference(dev, M, N, K_):
