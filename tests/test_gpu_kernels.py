@@ -898,6 +898,29 @@ def test_gemm_swiglu_few_rows_matches_fp32_reference(dev, M, F, K_):
     torch.testing.assert_close(out.float(), want, rtol=1e-2, atol=1e-2)   # values of size 1, one bf16 rounding
 
 
+@pytest.mark.parametrize("M", [64, 300])
+def test_gemm_swiglu_over_the_range_of_the_gate(dev, M):
+    """Gates from far below the range of exp to far above it, and infinities: silu tends to 0 and to the gate."""
+    from xccl_b200.ops import gemm
+    F = 1024
+    a = torch.zeros(M, 128, device=dev, dtype=torch.bfloat16)
+    a[:, 0] = 1
+    gate = torch.linspace(-130, 130, F, device=dev).to(torch.bfloat16)
+    gate[0], gate[-1] = -3e38, float("inf")
+    wg = torch.zeros(F, 128, device=dev, dtype=torch.bfloat16)
+    wg[:, 0] = gate
+    wu = torch.zeros_like(wg)
+    wu[:, 0] = 1
+    out = gemm.gemm_swiglu(a, wg, wu).double()
+    assert gemm.last_error() == 0
+    g = gate.double()
+    want = g / (1 + torch.exp(-g))
+    got, want = out[:, 1:-1], want[1:-1].expand(M, -1)
+    # half a unit of bf16 and what exp loses at 130 (2^-21 per unit of the exponent); below 2^-126 bf16 has steps of 2^-133
+    torch.testing.assert_close(got, want, rtol=2 ** -8, atol=2 ** -133)
+    assert bool((out[:, 0] == 0).all()) and bool((out[:, -1] == float("inf")).all())   # the gate is 1 x the weight
+
+
 @pytest.mark.parametrize("M", [1, 32, 33, 64, 65, 128])
 @pytest.mark.parametrize("N,K_", [(128, 128), (384, 1152), (1024, 8192)])
 def test_gemm_fp8_few_rows_matches_dequantised_reference(dev, M, N, K_):
