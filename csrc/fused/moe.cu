@@ -1,7 +1,7 @@
 // MoE expert dispatch / combine fused with the all-to-all (extension; the reference only has
 // alltoallv call sites: src/team_lib/nccl/xccl_nccl_collective.c:125-163).
 //
-// dispatch (ONE kernel): count tokens per expert, exchange the counts with every rank through
+// dispatch (ONE kernel; one rank alone has its own, without the exchange): count tokens per expert, exchange the counts with every rank through
 //   peer memory, turn them into receive offsets, and copy every routed token row straight into its
 //   slot of the destination rank's receive buffer - rows arrive grouped by (local expert, source
 //   rank), ready for a grouped GEMM. No host round trip, no intermediate permuted copy.
@@ -79,9 +79,21 @@ __device__ __forceinline__ void st_release_gpu(uint32_t *p, uint32_t v)
 }
 // Predicated 16-byte load that bypasses L1 (zeros when !on). A branch around the load instead makes the warp wait for
 // each load before it issues the next one.
-__device__ __forceinline__ uint4 ld16_if(const void *p, bool on)
+// kAlone: the memory is this GPU's and nobody writes it during the kernel.
+template <bool kAlone> __device__ __forceinline__ uint4 ld16_if(const void *p, bool on)
 {
     uint4 v = make_uint4(0, 0, 0, 0);
+    if (kAlone) {
+        asm volatile(
+            "{\n"
+            ".reg .pred q;\n"
+            "setp.ne.u32 q, %5, 0;\n"
+            "@q ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+            "}\n"
+            : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+            : "l"(p), "r"((uint32_t)on));
+        return v;
+    }
     asm volatile(
         "{\n"
         ".reg .pred q;\n"
@@ -295,10 +307,144 @@ __global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_kernel(MoeParams 
     }
 }
 
+// Exclusive prefix sum over the threads of a block of kMaxExperts; every thread calls it. *total: the sum of all.
+__device__ uint32_t block_prefix(uint32_t v, uint32_t *total)
+{
+    __shared__ uint32_t s_warp[32];
+    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+    uint32_t  incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_warp[wid] = incl;
+    __syncthreads();
+    uint32_t w = s_warp[lane];   // every warp adds the warps' sums up for itself
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
+    }
+    *total = __shfl_sync(0xffffffffu, w, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, w, wid > 0 ? wid - 1 : 0);
+    return incl - v + (wid > 0 ? before : 0);
+}
+
+// Dispatch of one rank alone. Every block routes for itself: it counts all entries per expert, those before its own tokens
+// apart, so that the first row of its entries of expert e is the prefix sum over the experts plus the entries of e before it.
+// No block waits for another (and the launch need not be cooperative); what every block reads besides its rows are the T x K
+// ids, from L2. Blocks own whole tokens; where there are fewer tokens than blocks, `parts` blocks share a token's row and
+// each derives the same rows for its entries. The first rows of x are on their way while the block counts.
+// One block that routed for all while the others waited: 128 tokens x 7168, 256 experts, top 8, 16.5 us, now 7.7; 16 tokens x
+// 2048 13.0 and 5.1; 4096 x 7168 (bound by 470 MB of stores) 112 and 104. With several ranks the counts have to be exchanged
+// anyway, and one block does it (moe_dispatch_kernel).
+constexpr int kOwnEntries = 1024;   // entries that a block routes at a time (callers: K <= kOwnEntries)
+
+__global__ void __launch_bounds__(kMaxExperts, 1) moe_dispatch_alone_kernel(MoeParams p)
+{
+    __shared__ uint32_t s_before[kMaxExperts], s_rest[kMaxExperts], s_row[kOwnEntries];
+    __shared__ int32_t  s_id[kOwnEntries];
+    const int      tid = threadIdx.x, lane = tid % 32, wid = tid / 32, nwarps = kMaxExperts / 32;
+    const int32_t *ids = p.ids[0];
+    const int      nent = p.T * p.K, blocks = gridDim.x;
+    const int      parts = max(1, blocks / p.T);
+    const int      part  = blocks >= p.T ? (int)blockIdx.x % parts : 0;
+    const int      t_lo  = blocks >= p.T ? min((int)blockIdx.x / parts, p.T) : (int)((long long)blockIdx.x * p.T / blocks);
+    const int      t_hi  = blocks >= p.T ? min(t_lo + 1, p.T) : (int)((long long)(blockIdx.x + 1) * p.T / blocks);
+    const uint32_t failed = *(volatile uint32_t *)p.error[0];   // by an earlier launch
+    // a warp takes seg_packs packs of a token's row at a time
+    const int      packs = p.H * 2 / 16, nseg = (packs + p.seg_packs - 1) / p.seg_packs;
+    const int      seg_lo = nseg * part / parts, segs = nseg * (part + 1) / parts - seg_lo;
+    auto load = [&](int t0, int it, uint4 (&v)[4]) {
+        const int    lo  = (seg_lo + it % segs) * p.seg_packs + lane, hi = min((seg_lo + it % segs + 1) * p.seg_packs, packs);
+        const uint4 *src = reinterpret_cast<const uint4 *>(p.x[0] + (size_t)(t0 + it / segs) * p.H);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (lo + 32 * u < hi) v[u] = __ldg(src + lo + 32 * u);
+        }
+    };
+    const int batch = max(1, kOwnEntries / p.K);   // tokens that are routed at a time
+    uint4     v[4];
+    if (wid < segs * min(batch, t_hi - t_lo)) load(t_lo, wid, v);
+
+    s_before[tid] = s_rest[tid] = 0;
+    __syncthreads();
+    // eight entries per thread in flight
+    for (int i0 = tid; i0 < nent; i0 += 8 * kMaxExperts) {
+        int e[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = i0 + u * kMaxExperts;
+            e[u]        = i < nent ? __ldg(ids + i) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (e[u] >= 0 && e[u] < p.E) atomicAdd((i0 + u * kMaxExperts < t_lo * p.K ? s_before : s_rest) + e[u], 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t before = s_before[tid], tot = before + s_rest[tid];
+    uint32_t       total;
+    const uint32_t first = block_prefix(tot, &total);
+    s_before[tid]        = first + before;   // the row of my next entry of expert tid
+    if (blockIdx.x == 0) {
+        if (tid < p.E) p.expert_rows[0][tid] = tot;
+        if (tid == 0) p.expert_rows[0][p.E] = total;
+        if (tid == 0 && total > (uint32_t)p.cap_rows) atomicExch(p.error[0], 0x400u);
+    }
+    if (total > (uint32_t)p.cap_rows || failed != 0) return;   // the same in every block: nobody writes
+    for (int t0 = t_lo; t0 < t_hi; t0 += batch) {
+        const int nt = min(batch, t_hi - t0), n = nt * p.K;
+        __syncthreads();
+        if (tid < n) s_id[tid] = __ldg(ids + (size_t)t0 * p.K + tid);
+        __syncthreads();
+        if (tid < n) {
+            const int32_t e   = s_id[tid];
+            uint32_t      row = 0xffffffffu;
+            if (e >= 0 && e < p.E) {
+                if (parts > 1) {   // one token: its earlier entries of the same expert, alike in every block
+                    row = s_before[e];
+                    for (int k = 0; k < tid; k++) row += s_id[k] == e;
+                } else {
+                    row = atomicAdd(s_before + e, 1u);
+                }
+                if (part == 0) {
+                    p.slot[0][(size_t)t0 * p.K + tid] = row;
+                    p.rsrc[0][row]                    = t0 + tid / p.K;
+                }
+            }
+            s_row[tid] = row;
+        }
+        __syncthreads();
+        for (int it = wid; it < nt * segs; it += nwarps) {
+            const int lo = (seg_lo + it % segs) * p.seg_packs + lane, hi = min((seg_lo + it % segs + 1) * p.seg_packs, packs);
+            const uint32_t *rows = s_row + it / segs * p.K;
+            uint4           next[4];
+            const int       nit = it + nwarps;
+            if (nit < nt * segs) load(t0, nit, next);
+            else if (t0 + batch < t_hi && wid < segs * min(batch, t_hi - t0 - batch)) load(t0 + batch, wid, next);
+            for (int k = 0; k < p.K; k++) {
+                const uint32_t row = rows[k];
+                if (row == 0xffffffffu) continue;
+                uint4 *dst = reinterpret_cast<uint4 *>(p.recv[0] + (size_t)row * p.H) + lo;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    if (lo + 32 * u < hi) dst[32 * u] = v[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = next[u];
+        }
+        // (a warp without an item in this batch has no load of the next one's on its way yet)
+        if (wid >= nt * segs && t0 + batch < t_hi && wid < segs * min(batch, t_hi - t0 - batch)) load(t0 + batch, wid, v);
+    }
+}
+
 // Block b meets block b of every rank before its first load (the peers' expert outputs are complete) and after its last
 // one (nobody's buffer is reused while a peer may still read it); the launch ends when all blocks have. One rank alone
 // has nobody to meet.
-__global__ void __launch_bounds__(1024, 1) moe_combine_kernel(MoeParams p)
+template <bool kAlone> __global__ void __launch_bounds__(1024, 1) moe_combine_kernel(MoeParams p)
 {
     const int local = blockIdx.y, rank = p.rank_base + local;
     const int EL    = p.E / p.tp;
@@ -309,72 +455,79 @@ __global__ void __launch_bounds__(1024, 1) moe_combine_kernel(MoeParams p)
         ok    = cross_rank_barrier(p, rank, blockIdx.x, epoch);
         if (!ok && threadIdx.x == 0) atomicExch(p.error[local], 0x403u);
     }
-    if (ok && *(volatile uint32_t *)p.error[local] == 0) {
-        // a warp adds up seg_packs packs of one token: lane k holds routing entry k, the warp shares the rows' addresses,
-        // and all (up to eight) expert rows of a pack are in flight at once. 4096 x 7168, top 8 (530 MB): 244 us with a
-        // warp per whole token and a branch per load, which made the eight loads wait for one another.
-        const int    lane = threadIdx.x % 32;
-        const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32, nwarps = (size_t)gridDim.x * blockDim.x / 32;
-        const int    packs = p.H * 2 / 16, nseg = (packs + p.seg_packs - 1) / p.seg_packs;
-        const size_t items = (size_t)p.T * nseg;
-        for (size_t it = warp; it < items; it += nwarps) {
-            const size_t t  = it / nseg;
-            const int    lo = (int)(it % nseg) * p.seg_packs, hi = min(lo + p.seg_packs, packs);
-            // routing entries of this token, eight at a time
-            // (with more than eight entries the running sum passes through bf16 between groups)
-            for (int kb = 0; kb < p.K; kb += 8) {
-                const int kn = min(8, p.K - kb);
-                unsigned long long my_row = 0;
-                float              my_g   = 0.0f;
-                if (lane < kn) {
-                    const size_t   i   = t * p.K + kb + lane;
-                    const int      e   = p.ids[local][i];
-                    const float    g   = p.w[local][i];
-                    const uint32_t row = p.slot[local][i];
-                    if (e >= 0 && e < p.E) {
-                        my_g   = g;
-                        my_row = (unsigned long long)(p.yout[e / EL] + (size_t)row * p.H);
+    // a warp adds up seg_packs packs of one token: lane k holds routing entry k, the warp shares the rows' addresses, and all
+    // (up to eight) expert rows of a pack are in flight at once. 4096 x 7168, top 8 (530 MB): 244 us with a warp per whole
+    // token and a branch per load, which made the eight loads wait for one another. The entries of a warp's next piece are
+    // loaded beside the rows of this one, and one rank alone reads without system scope: 104 us, now 97.
+    const int    lane = threadIdx.x % 32;
+    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32, nwarps = (size_t)gridDim.x * blockDim.x / 32;
+    const int    packs = p.H * 2 / 16, nseg = (packs + p.seg_packs - 1) / p.seg_packs;
+    const size_t items = ok ? (size_t)p.T * nseg : 0;
+    // entry kb + lane of a token (lanes 0-7): expert (-1: none), gate, row
+    auto entry = [&](size_t t, int kb, int &e, float &g, uint32_t &row) {
+        e   = -1;
+        g   = 0.0f;
+        row = 0;
+        if (lane < min(8, p.K - kb)) {
+            const size_t i = t * p.K + kb + lane;
+            e   = __ldg(p.ids[local] + i);
+            g   = __ldg(p.w[local] + i);
+            row = __ldg(p.slot[local] + i);
+        }
+    };
+    const uint32_t failed = *(volatile uint32_t *)p.error[local];
+    int      e_next = -1;
+    float    g_next = 0.0f;
+    uint32_t r_next = 0;
+    if (warp < items) entry(warp / nseg, 0, e_next, g_next, r_next);
+    for (size_t it = warp; it < items && failed == 0; it += nwarps) {
+        const size_t t  = it / nseg;
+        const int    lo = (int)(it % nseg) * p.seg_packs, hi = min(lo + p.seg_packs, packs);
+        // (with more than eight entries the running sum passes through bf16 between groups)
+        for (int kb = 0; kb < p.K; kb += 8) {
+            const bool     on     = e_next >= 0 && e_next < p.E;
+            const float    my_g   = on ? g_next : 0.0f;
+            const unsigned long long my_row = on ? (unsigned long long)(p.yout[kAlone ? 0 : e_next / EL] + (size_t)r_next * p.H) : 0ull;
+            if (kb + 8 < p.K) entry(t, kb + 8, e_next, g_next, r_next);
+            else if (it + nwarps < items) entry((it + nwarps) / nseg, 0, e_next, g_next, r_next);
+            const uint4 *rows[8];
+            float        gs[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                rows[k] = reinterpret_cast<const uint4 *>(__shfl_sync(0xffffffffu, my_row, k));
+                gs[k]   = __shfl_sync(0xffffffffu, my_g, k);
+            }
+            for (int k0 = lo + lane; k0 < hi; k0 += 32) {
+                uint4 raw[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) raw[k] = ld16_if<kAlone>(rows[k] + k0, rows[k] != nullptr);
+                float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                uint4 *dst = reinterpret_cast<uint4 *>(p.out[local] + t * p.H) + k0;
+                if (kb > 0) {
+                    const uint4 prev = *dst;
+                    const __nv_bfloat162 *ph = reinterpret_cast<const __nv_bfloat162 *>(&prev);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        float2 f = __bfloat1622float2(ph[j]);
+                        acc[2 * j] = f.x;
+                        acc[2 * j + 1] = f.y;
                     }
                 }
-                const uint4 *rows[8];
-                float        gs[8];
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
-                    rows[k] = reinterpret_cast<const uint4 *>(__shfl_sync(0xffffffffu, my_row, k));
-                    gs[k]   = __shfl_sync(0xffffffffu, my_g, k);
-                }
-                for (int k0 = lo + lane; k0 < hi; k0 += 32) {
-                    uint4 raw[8];
+                    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[k]);
 #pragma unroll
-                    for (int k = 0; k < 8; k++) raw[k] = ld16_if(rows[k] + k0, rows[k] != nullptr);
-                    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                    uint4 *dst = reinterpret_cast<uint4 *>(p.out[local] + t * p.H) + k0;
-                    if (kb > 0) {
-                        const uint4 prev = *dst;
-                        const __nv_bfloat162 *ph = reinterpret_cast<const __nv_bfloat162 *>(&prev);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            float2 f = __bfloat1622float2(ph[j]);
-                            acc[2 * j] = f.x;
-                            acc[2 * j + 1] = f.y;
-                        }
+                    for (int j = 0; j < 4; j++) {
+                        float2 f = __bfloat1622float2(h[j]);
+                        acc[2 * j] += gs[k] * f.x;
+                        acc[2 * j + 1] += gs[k] * f.y;
                     }
-#pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[k]);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            float2 f = __bfloat1622float2(h[j]);
-                            acc[2 * j] += gs[k] * f.x;
-                            acc[2 * j + 1] += gs[k] * f.y;
-                        }
-                    }
-                    uint4 o;
-                    __nv_bfloat162 *oh = reinterpret_cast<__nv_bfloat162 *>(&o);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                    *dst = o;
                 }
+                uint4 o;
+                __nv_bfloat162 *oh = reinterpret_cast<__nv_bfloat162 *>(&o);
+#pragma unroll
+                for (int j = 0; j < 4; j++) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+                *dst = o;
             }
         }
     }
@@ -530,6 +683,7 @@ xccl_status_t xccl_moe_dispatch(xccl_moe_ws_h w, const void *const *x, const int
         w->p.x[l]   = (const __nv_bfloat16 *)x[l];
         w->p.ids[l] = ids[l];
     }
+    if (w->p.tp == 1 && w->p.K <= kOwnEntries) return launch(moe_dispatch_alone_kernel, w, w->blocks, false, (cudaStream_t)stream);
     return launch(moe_dispatch_kernel, w, w->blocks, true, (cudaStream_t)stream);
 }
 
@@ -544,7 +698,7 @@ xccl_status_t xccl_moe_combine(xccl_moe_ws_h w, const int32_t *const *ids, const
     }
     // several ranks: a row of barrier flags per block
     const int blocks = w->p.tp > 1 ? std::min(w->blocks, nvl::kMaxBlocks) : w->blocks;
-    return launch(moe_combine_kernel, w, blocks, w->p.tp > 1, (cudaStream_t)stream);
+    return launch(w->p.tp > 1 ? moe_combine_kernel<false> : moe_combine_kernel<true>, w, blocks, w->p.tp > 1, (cudaStream_t)stream);
 }
 
 void *xccl_moe_ws_buffer(xccl_moe_ws_h w, int local_rank, int which)

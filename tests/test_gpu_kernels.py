@@ -776,6 +776,49 @@ def test_moe_row_pieces_many_entries_and_dropped_ids(dev, ranks, T, H, E, Kk):
         ws.close()
 
 
+@pytest.mark.parametrize("T,H,E,Kk", [
+    (1, 8, 4, 3), (1, 4104, 16, 8),                  # more blocks than pieces of the one row, and fewer
+    (40, 1032, 8, 6), (147, 264, 16, 5),             # several blocks and one block per token
+    (149, 264, 1024, 8), (700, 520, 16, 4),          # a few tokens per block
+    (6000, 8, 64, 64), (300, 16, 8, 1000),           # more entries than a block routes at a time
+    (5, 16, 8, 1500),                                # more entries per token than that: the kernel of several ranks
+])
+def test_moe_one_rank_with_repeated_experts(dev, T, H, E, Kk):
+    """One rank alone, entries of a token that name the same expert again and again: rows grouped by expert, each entry with
+    a row of its own, and the row that dispatch wrote is the one that combine reads."""
+    from xccl_b200.ops.moe import MoeWorkspace
+    ws = MoeWorkspace(T, H, E, Kk)
+    try:
+        g = torch.Generator(device=dev).manual_seed(T * 7 + Kk)
+        x = torch.randn(T, H, device=dev, generator=g).to(torch.bfloat16)
+        ids = torch.randint(-1, E + 1, (T, Kk), device=dev, generator=g).to(torch.int32)   # -1 and E: dropped
+        gates = torch.rand(T, Kk, device=dev, generator=g) / Kk
+        for _ in range(2):
+            ws.dispatch([x], [ids])
+        assert ws.error() == 0
+        valid = (ids >= 0) & (ids < E)
+        rows = ws.expert_rows().long()
+        n = int(valid.sum())
+        assert torch.equal(rows[:E], torch.bincount(ids[valid].long(), minlength=E)) and int(rows[E]) == n
+        src = ws.row_source()[:n].long()
+        e = torch.repeat_interleave(torch.arange(E, device=dev), rows[:E])
+        assert torch.equal(ws.recv()[:n], x[src])
+        asked = (ids.long() * T + torch.arange(T, device=dev)[:, None])[valid]
+        assert torch.equal((e * T + src).sort().values, asked.sort().values)
+        # experts: multiples of the row by a power of two, exact in bf16
+        mult = torch.tensor([1.0, 0.5, 2.0, 0.25], device=dev)
+        ws.expert_out()[:n] = (ws.recv()[:n].float() * mult[e % 4][:, None]).to(torch.bfloat16)
+        out = torch.full((T, H), 5.0, dtype=torch.bfloat16, device=dev)
+        ws.combine([ids], [gates], [out])
+        assert ws.error() == 0
+        f = (gates.double() * mult[ids.long() % 4].double() * valid).sum(-1, keepdim=True)
+        # every eight entries the running sum is rounded to bf16: half of its spacing (2^-8) of a sum that only grows
+        bound = (-(-Kk // 8) * 1.03 * 2.0 ** -8 + 1e-5) * (f * x.double().abs())
+        assert bool(((out.double() - f * x.double()).abs() <= bound).all())
+    finally:
+        ws.close()
+
+
 @pytest.mark.parametrize("ranks", [1, 2, 4])
 def test_moe_receive_buffer_too_small(dev, ranks):
     """One rank's receive buffer is a row too small: every rank reports it, nobody writes a row, and the ranks meet at the
