@@ -8,7 +8,7 @@
 // of weight loads in flight. Measured on one B200, operands in DRAM, before (large kernel with 256-column tiles) and now: bf16
 // 16 x 8192 x 8192 (134 MB of weights) 47.5 -> 26.5 us, 128 x 8192 x 8192 49.0 -> 34.2 us; SwiGLU 16 x 3584 x 8192 69.0 ->
 // 26.2 us; fp8 64 x 7168 x 8192 49.2 -> 18.6 us.
-// The line lies at the 128 rows that one MMA holds. On both sides of it at 128 rows, this kernel / the large one with the
+// One MMA holds 128 rows; more of them come in several blocks where that pays (skinny_plan_rows). On both sides of the line at 128 rows, this kernel / the large one with the
 // narrower tiles it now has, L2 flushed, event times in steps of 2 us: bf16 N 8192, K 8192 40.9 / 53.2, K 2048 20.5 / 20.7,
 // K 512 15.7 / 14.6; N 2048, K 1024 16.3 / 14.5 (K up to 1024 is where the large one is level or up to 2 us ahead); SwiGLU N
 // 8192, K 2048 37 / 50; fp8 N 8192, K 2048 19 / 26, N 28672, K 512 22.3 / 20.6.
@@ -92,6 +92,8 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
 
     const int  warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int  split = blockIdx.x, tile = blockIdx.y;  // split = rank in the cluster
+    const int  m0   = (int)blockIdx.z * mn;            // first token of this block of rows
+    const int  rows = min(p.M - m0, mn);
     const int  kb_lo = (int)((long)split * p.plan.kblocks / p.plan.splits);
     const int  kb_hi = (int)((long)(split + 1) * p.plan.kblocks / p.plan.splits);
     AbortFlag  ab{&s_abort, p.error, p.budget_ns};
@@ -130,7 +132,8 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
 
     if (warp == 0) {
         if (elect_one()) {
-            const uint64_t pol_w = l2_policy_evict_first(), pol_a = l2_policy_evict_last();
+            // (several blocks of rows read the same weights at about the same time)
+            const uint64_t pol_a = l2_policy_evict_last(), pol_w = gridDim.z == 1 ? l2_policy_evict_first() : pol_a;
             int      s = 0;
             uint32_t phase = 0;
             int      issued = 0;
@@ -144,7 +147,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                 mbar_arrive_expect_tx(full_bar(s), stage_bytes);
                 tma_load_2d_hint(st, &maps.b0, kb * kKE, tile * 128, full_bar(s), pol_w);
                 if (kSwi) tma_load_2d_hint(st + kWBytes, &maps.b1, kb * kKE, tile * 128, full_bar(s), pol_w);
-                tma_load_2d_hint(st + kMats * kWBytes, &maps.a, kb * kKE, 0, full_bar(s), pol_a);
+                tma_load_2d_hint(st + kMats * kWBytes, &maps.a, kb * kKE, m0, full_bar(s), pol_a);
                 issued++;
                 if (++s == stages) {
                     s = 0;
@@ -218,7 +221,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                 uu0[i] = __ldg(w0 + kb);
                 uu1[i] = __ldg(w1 + kb);
 #pragma unroll
-                for (int j = 0; j < kNT; j++) xx[i][j] = __ldcg(p.sa + (size_t)min(lane + 32 * j, p.M - 1) * kbn + kb);
+                for (int j = 0; j < kNT; j++) xx[i][j] = __ldcg(p.sa + (size_t)(m0 + min(lane + 32 * j, rows - 1)) * kbn + kb);
             }
         };
         int      slot = 0;
@@ -326,7 +329,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
         cluster_sync_all();  // every CTA's partial sums of the round can be read
         if (epi) {
             const int tid = threadIdx.x - 64, nthr = kEpiWarps * 32;
-            const int tokens = min(t1, p.M) - t0;
+            const int tokens = min(t1, rows) - t0;
             const int mine   = tokens > split ? (tokens - split + p.plan.splits - 1) / p.plan.splits : 0;
             // sixteen lanes share a token of 128 outputs, eight outputs each
             for (int it = tid; it < mine * 16; it += nthr) {
@@ -365,7 +368,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
 #pragma unroll
                     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(mask, amax, o));
                     const float sc = fmaxf(amax, 1e-12f) / 448.0f, inv = 1.0f / sc;
-                    if (q == 0) p.out_scale[(size_t)(t0 + t) * (size_t)(p.N / 128) + tile] = sc;
+                    if (q == 0) p.out_scale[(size_t)(m0 + t0 + t) * (size_t)(p.N / 128) + tile] = sc;
                     uint32_t w2[2];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -374,9 +377,9 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                                 ((uint32_t)__nv_cvt_float_to_fp8(x[0][4 * h + 2] * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
                                 ((uint32_t)__nv_cvt_float_to_fp8(x[0][4 * h + 3] * inv, __NV_SATFINITE, __NV_E4M3) << 24);
                     }
-                    *reinterpret_cast<uint2 *>((uint8_t *)p.C + (size_t)(t0 + t) * p.ldc + col) = make_uint2(w2[0], w2[1]);
+                    *reinterpret_cast<uint2 *>((uint8_t *)p.C + (size_t)(m0 + t0 + t) * p.ldc + col) = make_uint2(w2[0], w2[1]);
                 } else if (col < p.N) {
-                    *reinterpret_cast<uint4 *>((__nv_bfloat16 *)p.C + (size_t)(t0 + t) * p.ldc + col) =
+                    *reinterpret_cast<uint4 *>((__nv_bfloat16 *)p.C + (size_t)(m0 + t0 + t) * p.ldc + col) =
                         make_uint4(pack_bf16x2(x[0][0], x[0][1]), pack_bf16x2(x[0][2], x[0][3]),
                                    pack_bf16x2(x[0][4], x[0][5]), pack_bf16x2(x[0][6], x[0][7]));
                 }
@@ -433,7 +436,7 @@ template <typename F> int placeable(int splits, F &&fits)
 void launch_config(const SkinnyPlan &plan, bool fp8, cudaStream_t stream, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr)
 {
     *cfg = cudaLaunchConfig_t{};
-    cfg->gridDim          = dim3((unsigned)plan.splits, (unsigned)plan.tiles);
+    cfg->gridDim          = dim3((unsigned)plan.splits, (unsigned)plan.tiles, (unsigned)plan.blocks);
     cfg->blockDim         = dim3(fp8 ? kSkinnyThreadsFp8 : kSkinnyThreads);
     cfg->dynamicSmemBytes = (size_t)plan.smem_bytes;
     cfg->stream           = stream;
@@ -509,11 +512,13 @@ int skinny_share(int tiles, int kblocks, int occ, int sms)
 
 }  // namespace
 
-bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
+// A plan for `blocks` blocks of up to M rows.
+static bool plan_blocks(int M, int blocks, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
 {
     if (M <= 0 || M > kSkinnyMaxM || N <= 0 || K <= 0) return false;
     SkinnyPlan  q{};
     const int   mats = swiglu ? 2 : 1;
+    q.blocks  = blocks;
     q.mn      = fp8 ? (M <= 32 ? 32 : M <= 64 ? 64 : 128) : (M + 15) / 16 * 16;
     q.tiles   = (N + 127) / 128;
     q.kblocks = (K + (fp8 ? 127 : 63)) / (fp8 ? 128 : 64);
@@ -526,7 +531,7 @@ bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan
     q.cols    = mats * (fp8 ? q.mn : (q.mn + 31) / 32 * 32);
     q.nbuf    = fp8 ? std::max(1, std::min(kMaxBuf, 512 / occ / q.cols)) : 1;
     q.tmem_cols = pow2_at_least(q.nbuf * q.cols, 32);
-    q.splits  = skinny_share(q.tiles, q.kblocks, occ, sms);
+    q.splits  = skinny_share(q.tiles * blocks, q.kblocks, occ, sms);
     q.chunk   = std::min(q.mn, q.stages * stage / (512 * mats) / 16 * 16);
     q.smem_bytes = fixed + q.stages * stage;
     if (q.stages < 2 || q.chunk < 16) return false;
@@ -534,14 +539,40 @@ bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan
     return true;
 }
 
+bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
+{
+    return plan_blocks(M, 1, N, K, fp8, swiglu, sms, out);
+}
+
+// Rows beyond one MMA, in blocks of up to 128: where the tiles of the large kernel (256 x 256, in bf16 narrower ones too) leave
+// most of the chip idle, small tiles whose K is shared by a cluster fill it, although each block of rows reads the weights
+// again (from L2). fp8: as long as every CTA has an SM to itself (the large kernel's fp8 tiles are all 256 columns wide), with
+// SwiGLU only where CTAs share K. bf16: where at least three CTAs share 24 K blocks and more; with fewer it is level or behind,
+// and SwiGLU stays with the large kernel. Large / few-rows kernel, 140 products each of 129 to 1536 rows, N and K from 256 to
+// 8192, L2 flushed: fp8 within the rule 1.50 times faster on average, 1.14 the least (outside 0.6 to 1.0), bf16 1.30 and 0.95
+// (outside 0.91 on average), bf16 SwiGLU 0.89 where the CTAs fit the SMs. fp8 212 x 768 x 7808 54.3 / 20.5 us, 502 x 1664 x 5376
+// 37.9 / 22.5, 8192 x 256 x 512 17.3 / 12.3; bf16 143 x 2928 x 7728 39.9 / 28.7, 370 x 304 x 5216 27.5 / 18.5. fp8 block step (SwiGLU and
+// down projection) 256 rows, 1152, 4352 64.5 / 44.0, 512 rows, 5376, 2944 76.8 (97.2 with unshared SwiGLU tiles).
+bool skinny_plan_rows(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
+{
+    if (M <= kSkinnyMaxM) return skinny_plan(M, N, K, fp8, swiglu, sms, out);
+    const int blocks = (M - 1) / kSkinnyMaxM + 1;
+    if ((swiglu && !fp8) || blocks > sms) return false;
+    SkinnyPlan q{};
+    if (!plan_blocks((M - 1) / blocks + 1, blocks, N, K, fp8, swiglu, sms, &q)) return false;
+    if (fp8 ? q.blocks * q.tiles * q.splits > sms || (swiglu && q.splits < 2) : q.splits < 3 || q.kblocks < 24) return false;
+    *out = q;
+    return true;
+}
+
 bool try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st)
 {
     // what the large kernels refuse is left to them to refuse
-    if (a.M > kSkinnyMaxM || (a.fp8 ? (a.K % 128 != 0 || a.N % 128 != 0) : (a.K % 8 != 0 || a.N % 8 != 0))) return false;
+    if ((a.fp8 ? (a.K % 128 != 0 || a.N % 128 != 0) : (a.K % 8 != 0 || a.N % 8 != 0))) return false;
     int        dev = 0, sms = 0;
     SkinnyPlan plan;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-    if (!skinny_plan(a.M, a.N, a.K, a.fp8, a.swiglu, sms, &plan)) return false;
+    if (!skinny_plan_rows(a.M, a.N, a.K, a.fp8, a.swiglu, sms, &plan)) return false;
     *st = launch_skinny(a, plan, stream);
     if (*st == XCCL_OK) return true;
     (void)cudaGetLastError();   // refused: the large kernel serves the call, or says why not
@@ -591,13 +622,22 @@ extern "C" int xccl_tp_skinny_cluster(int splits, unsigned fits)
 }
 
 // Host-side view of the cut (tests): out = {mn, tiles, splits, kblocks, stages, nbuf, cols, tmem_cols, chunk, smem_bytes,
-// CTAs per SM}. Returns 1 when the sizes are served by this kernel, 0 otherwise.
-extern "C" int xccl_tp_skinny_plan(int M, int N, int K, int fp8, int swiglu, int sms, int *out)
+// CTAs per SM}. Returns the number of blocks of rows (here 1), 0 when the sizes are not for this kernel.
+static int skinny_plan_out(bool rows, int M, int N, int K, bool fp8, bool swiglu, int sms, int *out)
 {
     xccl::tp::SkinnyPlan q;
-    if (out == nullptr || !xccl::tp::skinny_plan(M, N, K, fp8 != 0, swiglu != 0, sms, &q)) return 0;
+    if (out == nullptr || !(rows ? xccl::tp::skinny_plan_rows : xccl::tp::skinny_plan)(M, N, K, fp8, swiglu, sms, &q)) return 0;
     const int v[11] = {q.mn, q.tiles, q.splits, q.kblocks, q.stages, q.nbuf, q.cols, q.tmem_cols, q.chunk, q.smem_bytes,
-                       xccl::tp::skinny_occupancy(q.mn, fp8 != 0, swiglu != 0)};
+                       xccl::tp::skinny_occupancy(q.mn, fp8, swiglu)};
     std::copy(v, v + 11, out);
-    return 1;
+    return q.blocks;
+}
+extern "C" int xccl_tp_skinny_plan(int M, int N, int K, int fp8, int swiglu, int sms, int *out)
+{
+    return skinny_plan_out(false, M, N, K, fp8 != 0, swiglu != 0, sms, out);
+}
+// The same for any number of rows: returns the number of blocks of rows, 0 when the large kernel serves the product.
+extern "C" int xccl_tp_skinny_plan_rows(int M, int N, int K, int fp8, int swiglu, int sms, int *out)
+{
+    return skinny_plan_out(true, M, N, K, fp8 != 0, swiglu != 0, sms, out);
 }

@@ -1,4 +1,5 @@
-// GEMM for few rows of activations (decoding): C[M,N] = A[M,K] * B[N,K]^T with M <= kSkinnyMaxM, plain or SwiGLU, bf16 or
+// GEMM for few rows of activations (decoding; more rows where the large kernel's tiles would leave the chip idle): C[M,N] =
+// A[M,K] * B[N,K]^T in blocks of up to kSkinnyMaxM rows, plain or SwiGLU, bf16 or
 // block-scaled fp8 (same operands, scales and rounding as the kernels of tp_gemm.cuh). Implemented in tp_skinny.cu.
 #pragma once
 #include <cuda_runtime.h>
@@ -23,7 +24,8 @@ struct SkinnyArgs {
 
 // How a launch is cut up (a pure function of the sizes; the tests walk it on the CPU).
 struct SkinnyPlan {
-    int mn;        // columns of the MMA: M rounded up
+    int mn;        // columns of the MMA: rows of a block rounded up
+    int blocks;    // blocks of rows (each up to kSkinnyMaxM)
     int tiles;     // blocks of 128 weight rows
     int splits;    // CTAs of a cluster that share the K blocks of a tile
     int kblocks;
@@ -36,6 +38,8 @@ struct SkinnyPlan {
 };
 // False when the sizes are not for this kernel (the callers then use launch_gemm / launch_gemm_fp8).
 bool          skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *plan);
+// The same for any number of rows (blocks of them): false also where the large kernel is the faster one.
+bool          skinny_plan_rows(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *plan);
 // Runs the product here when its sizes are for this kernel and the device takes the launch (true); otherwise nothing has
 // been launched and the caller's large kernel serves it.
 bool          try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st);

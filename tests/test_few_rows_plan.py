@@ -79,3 +79,34 @@ def test_tiles_run_in_one_wave_of_the_clusters_a_gpu_holds(fp8, swiglu):
     (64, 2048, 8192, True, False, 4), (16, 1024, 8192, False, False, 8), (128, 28672, 8192, False, True, 1)])
 def test_share_at_the_measured_sizes(M, N, K_, fp8, swiglu, splits):
     assert _plan(M, N, K_, fp8, swiglu)["splits"] == splits
+
+
+def _plan_rows(M, N, K_, fp8, swiglu, sms=148):
+    out = (C.c_int * len(FIELDS))()
+    fn = K.load().xccl_tp_skinny_plan_rows
+    fn.restype = C.c_int
+    n = fn(M, N, K_, int(fp8), int(swiglu), sms, out)
+    return dict(zip(FIELDS, out), blocks=n) if n else None
+
+
+@pytest.mark.parametrize("fp8,swiglu", [(False, False), (True, False), (True, True)])
+def test_blocks_of_rows_cover_the_rows_and_keep_to_the_rule(fp8, swiglu):
+    taken = 0
+    for M in (1, 128, 129, 200, 256, 257, 500, 1024, 1500, 4000, 8192):
+        for N in (128, 384, 1024, 2944, 7168):
+            for K_ in (128, 512, 1536, 4096, 8192):
+                p = _plan_rows(M, N, K_, fp8, swiglu)
+                if M <= 128:
+                    assert p is not None and p.pop("blocks") == 1 and p == _plan(M, N, K_, fp8, swiglu)
+                    continue
+                if p is None:
+                    continue
+                taken += 1
+                # every row in one block, no block without rows, and as many CTAs as the measured rule allows
+                assert p["mn"] <= 128 and (p["blocks"] - 1) * p["mn"] < M <= p["blocks"] * p["mn"]
+                ctas = p["blocks"] * p["tiles"] * p["splits"]
+                assert p["splits"] >= (1 if fp8 and not swiglu else 2 if fp8 else 3)
+                assert ctas <= 148 if fp8 else p["kblocks"] >= 24 and ctas <= 2 * 148
+    assert taken > 20
+    assert _plan_rows(300, 1024, 8192, False, True) is None      # bf16 SwiGLU stays with the large kernel
+    assert _plan_rows(1 << 30, 128, 128, True, False) is None

@@ -893,10 +893,10 @@ def test_gemm_fp8_blockscaled_matches_dequantised_reference(dev, M, N, K_):
 
 
 @pytest.mark.parametrize("off", [0, 1])
-@pytest.mark.parametrize("M,N,K_", [(129, 128, 128), (130, 384, 256), (255, 256, 384), (513, 640, 512), (257, 128, 640), (300, 896, 1152)])
+@pytest.mark.parametrize("M,N,K_", [(1409, 1792, 128), (1290, 1920, 256), (2047, 1280, 384), (513, 4096, 512), (2049, 1408, 640), (1300, 1920, 1152)])
 def test_gemm_fp8_blockscaled_scale_groups(dev, M, N, K_, off):
     """Scales reach the kernel four K blocks at a time, 16 bytes per row where the rows are aligned: numbers of K blocks
-    around the groups, scales that do not start on 16 bytes, a last tile half outside N."""
+    around the groups, scales that do not start on 16 bytes, a last tile half outside N. (Sizes of the large kernel.)"""
     from xccl_b200.ops import gemm
     a = torch.randn(M, K_, device=dev) * torch.rand(M, 1, device=dev) * 3
     b = torch.randn(N, K_, device=dev) * 0.05 * torch.rand(N // 128, device=dev).repeat_interleave(128)[:, None]
@@ -939,6 +939,57 @@ def test_gemm_swiglu_few_rows_matches_fp32_reference(dev, M, F, K_):
     assert gemm.last_error() == 0
     want = torch.nn.functional.silu(a.float() @ wg.float().t()) * (a.float() @ wu.float().t())
     torch.testing.assert_close(out.float(), want, rtol=1e-2, atol=1e-2)   # values of size 1, one bf16 rounding
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("M,N,K_", [(129, 384, 2048), (255, 1024, 4096), (256, 512, 1536), (257, 128, 8192), (700, 256, 4224),
+                                    (1300, 384, 1664)])
+def test_gemm_blocks_of_few_rows(dev, fp8, M, N, K_):
+    """More rows than one MMA in the few-rows kernel: whole and ragged blocks of rows, CTAs that share K and that do not,
+    nothing written outside the output."""
+    from xccl_b200.ops import gemm
+    a = torch.randn(M, K_, device=dev) * (0.2 + torch.rand(M, 1, device=dev))
+    b = torch.randn(N, K_, device=dev) * 0.05
+    guard = torch.full((M + 2, N), 7.0, device=dev, dtype=torch.bfloat16)
+    if fp8:
+        a8, sa = gemm.quantize_act_1x128(a)
+        b8, sb = gemm.quantize_weight_128x128(b)
+        gemm.gemm_fp8_blockscaled(a8, sa, b8, sb, guard[1:M + 1])
+        a, b = gemm.dequantize(a8, sa, 1), gemm.dequantize(b8, sb, 128)
+    else:
+        a, b = a.to(torch.bfloat16), b.to(torch.bfloat16)
+        gemm.gemm_bf16(a, b, guard[1:M + 1])
+    assert gemm.last_error() == 0
+    want = a.double() @ b.double().t()
+    # half a unit in the last place of bf16 (2^-9), and 32-bit sums of K products far below the largest value
+    torch.testing.assert_close(guard[1:M + 1].double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+    assert bool((guard[0] == 7).all()) and bool((guard[M + 1] == 7).all())
+
+
+@pytest.mark.parametrize("tokens", [256, 384])
+def test_tp_mlp_fp8_blocks_of_few_rows(dev, tokens):
+    """The fp8 block on one rank with more rows than one MMA: SwiGLU with its quantised output and the down projection in
+    blocks of rows, against the dequantised block with the same rounding steps in between."""
+    from xccl_b200.models.tp_mlp import TpMlpFp8
+    from xccl_b200.ops import gemm
+    mlp = TpMlpFp8(tokens, 1024, 1536)
+    try:
+        x = torch.randn(tokens, 1024, device=dev).to(torch.bfloat16)
+        y = mlp.forward([x])[0]
+        mlp.check_error()
+        deq = lambda q, s: gemm.dequantize(q, s, 128).double()
+        xq = gemm.dequantize(mlp.x8[0], mlp.sx[0], 1).double()
+        g, u = xq @ deq(mlp.w_gate8[0], mlp.s_gate[0]).t(), xq @ deq(mlp.w_up8[0], mlp.s_up[0]).t()
+        h = g / (1 + torch.exp(-g)) * u
+        hq = gemm.dequantize(mlp.h8[0], mlp.sh[0], 1).double()
+        # the intermediate: half of an e4m3 spacing (2^-4 of a value; below the smallest normal 2^-10 in units of a 448th of the
+        # block's largest value, which is less than 2^-17 of it)
+        block = h.view(tokens, -1, 128).abs().amax(-1, keepdim=True).expand(-1, -1, 128).reshape(tokens, -1)
+        assert bool(((hq - h).abs() <= (2 ** -4 + 1e-3) * h.abs() + block * 2 ** -17).all())
+        want = hq @ deq(mlp.w_down8[0], mlp.s_down[0]).t()
+        torch.testing.assert_close(y.double(), want, rtol=2 ** -8, atol=1e-5 * float(want.abs().max()))
+    finally:
+        mlp.close()
 
 
 @pytest.mark.parametrize("M", [64, 300])
