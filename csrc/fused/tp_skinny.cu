@@ -87,8 +87,6 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
     auto empty_bar      = [&](int s) { return bars + 8u * (kMaxStages + s); };
     auto tmem_full_bar  = [&](int a) { return bars + 8u * (2 * kMaxStages + a); };
     auto tmem_empty_bar = [&](int a) { return bars + 8u * (2 * kMaxStages + kMaxBuf + a); };
-    auto sc_full_bar    = [&](int s) { return bars + 8u * (2 * kMaxStages + 2 * kMaxBuf + s); };
-    auto sc_empty_bar   = [&](int s) { return bars + 8u * (2 * kMaxStages + 2 * kMaxBuf + kScaleSlots + s); };
 
     const int  warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int  split = blockIdx.x, tile = blockIdx.y;  // split = rank in the cluster
@@ -105,12 +103,8 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < nbuf; a++) {
-            mbar_init(tmem_full_bar(a), 1);
+            mbar_init(tmem_full_bar(a), kFp8 ? 2 : 1);  // fp8: the product and its scales
             mbar_init(tmem_empty_bar(a), kEpiWarps);
-        }
-        for (int s = 0; kFp8 && s < kScaleSlots; s++) {
-            mbar_init(sc_full_bar(s), 1);
-            mbar_init(sc_empty_bar(s), kEpiWarps);
         }
         mbar_fence_init();
         tma_prefetch_desc(&maps.a);
@@ -172,8 +166,8 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
             uint32_t phase = 0, acc_phase = 0;
             bool     ok = true;
             for (int kb = kb_lo; kb < kb_hi && ok; kb++) {
-                if (kFp8 && !mbar_wait(tmem_empty_bar(a), acc_phase ^ 1, ab, 3)) break;
                 if (!mbar_wait(full_bar(s), phase, ab, 4)) break;
+                if (kFp8 && !mbar_wait(tmem_empty_bar(a), acc_phase ^ 1, ab, 3)) break;
                 tc_fence_after();
                 const uint32_t st = ring + s * stage_bytes;
                 const uint64_t dt = make_desc_sw128(st + kMats * kWBytes);
@@ -190,7 +184,6 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                         }
                     }
                 }
-                mma_commit(empty_bar(s));
                 if (kFp8) {
                     mma_commit(tmem_full_bar(a));
                     if (++a == nbuf) {
@@ -198,6 +191,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                         acc_phase ^= 1;
                     }
                 }
+                mma_commit(empty_bar(s));
                 if (++s == stages) {
                     s = 0;
                     phase ^= 1;
@@ -209,7 +203,10 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
     } else if (kFp8 && warp == 2 + kEpiWarps) {
         // activation scale x weight scale of every token for the K blocks ahead. The loads are unconditional (clamped) and
         // those of the next four K blocks are in flight while this group's products are handed over: their latency from
-        // DRAM is about two K blocks' share of the time.
+        // DRAM is about two K blocks' share of the time. A product buffer counts as full when its scales are there too, so the
+        // promotion warps wait once per K block. Product n's scales are written when product n - nbuf and its scales are
+        // complete: then everybody has emptied n - 2 nbuf, and the slot's last reader was n - kScaleSlots.
+        static_assert(kScaleSlots >= 2 * kMaxBuf, "a slot's last reader has finished");
         constexpr int kNT = kCW > 0 ? kCW / 16 : 1;  // tokens per lane
         const int    kbn = p.plan.kblocks;
         const float *w0  = p.sb0 + (size_t)tile * kbn, *w1 = kSwi ? p.sb1 + (size_t)tile * kbn : w0;
@@ -224,7 +221,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                 for (int j = 0; j < kNT; j++) xx[i][j] = __ldcg(p.sa + (size_t)(m0 + min(lane + 32 * j, rows - 1)) * kbn + kb);
             }
         };
-        int      slot = 0;
+        int      slot = 0, a = 0;
         uint32_t phase = 0;
         bool     ok = true;
         load_group(kb_lo, x[0], u0[0], u1[0]);
@@ -235,7 +232,7 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
 #pragma unroll
                 for (int i = 0; i < kScaleGroup; i++) {
                     if (g + h * kScaleGroup + i >= kb_hi || !ok) continue;
-                    ok = mbar_wait(sc_empty_bar(slot), phase ^ 1, ab, 7);
+                    ok = mbar_wait(tmem_full_bar(a), phase ^ 1, ab, 7);
                     float *dst = scales + slot * kMats * mn;
 #pragma unroll
                     for (int j = 0; j < kNT; j++) {
@@ -243,55 +240,60 @@ skinny_kernel(SkinnyParams p, const __grid_constant__ SkinnyMaps maps)
                         if (kSwi) dst[mn + lane + 32 * j] = x[h][i][j] * u1[h][i];
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(sc_full_bar(slot));
-                    if (++slot == kScaleSlots) {
-                        slot = 0;
+                    if (lane == 0 && ok) mbar_arrive(tmem_full_bar(a));
+                    if (++slot == kScaleSlots) slot = 0;
+                    if (++a == nbuf) {
+                        a = 0;
                         phase ^= 1;
                     }
                 }
             }
         }
     } else if (kFp8) {
+        // What bounds the loop is its serial chain: all of a chunk's columns and scales are on their way before the first is
+        // waited for, and there is one wait per K block (with one for the scales beside it and sixteen columns at a time 64 x 7168
+        // x 8192 took 18.5 us, now 17.8, the block step of 128 tokens, 8192, 14336 115.7, now 110.3).
+        constexpr int kB = kMats * kCW > 64 || kCW < 32 ? 16 : 32;   // columns (tokens) at a time
         int      a = 0, slot = 0;
-        uint32_t acc_phase = 0, sc_phase = 0;
+        uint32_t acc_phase = 0;
 #pragma unroll
         for (int j = 0; j < kMats * kCW; j++) acc[j] = 0.0f;
         for (int kb = kb_lo; kb < kb_hi; kb++) {
-            if (!mbar_wait(sc_full_bar(slot), sc_phase, ab, 8) || !mbar_wait(tmem_full_bar(a), acc_phase, ab, 5)) break;
+            if (!mbar_wait(tmem_full_bar(a), acc_phase, ab, 5)) break;
             tc_fence_after();
             const float   *sc = scales + slot * kMats * mn + half * kCW;
             const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * p.plan.cols + half * kCW);
 #pragma unroll
             for (int m = 0; m < kMats; m++) {
 #pragma unroll
-                for (int c = 0; c < kCW; c += 16) {
-                    uint32_t v[16];
-                    tmem_ld_32x16(t0 + m * (p.plan.cols / kMats) + c, v);
-                    tmem_ld_wait();
+                for (int c = 0; c < kCW; c += kB) {
+                    uint32_t v[kB / 16][16];
+                    float4   f[kB / 4];
 #pragma unroll
-                    for (int e = 0; e < 16; e += 4) {
-                        const float4 f = *reinterpret_cast<const float4 *>(sc + m * mn + c + e);
-                        acc[m * kCW + c + e]     = fmaf(f.x, __uint_as_float(v[e]), acc[m * kCW + c + e]);
-                        acc[m * kCW + c + e + 1] = fmaf(f.y, __uint_as_float(v[e + 1]), acc[m * kCW + c + e + 1]);
-                        acc[m * kCW + c + e + 2] = fmaf(f.z, __uint_as_float(v[e + 2]), acc[m * kCW + c + e + 2]);
-                        acc[m * kCW + c + e + 3] = fmaf(f.w, __uint_as_float(v[e + 3]), acc[m * kCW + c + e + 3]);
+                    for (int b = 0; b < kB / 16; b++) tmem_ld_32x16(t0 + m * (p.plan.cols / kMats) + c + 16 * b, v[b]);
+#pragma unroll
+                    for (int e = 0; e < kB / 4; e++) f[e] = *reinterpret_cast<const float4 *>(sc + m * mn + c + 4 * e);
+#pragma unroll
+                    for (int b = 0; b < kB / 16; b++) tmem_ld_wait_16(v[b]);
+#pragma unroll
+                    for (int e = 0; e < kB; e += 4) {
+                        const uint32_t *x = v[e / 16] + e % 16;
+                        float          *s = acc + m * kCW + c + e;
+                        s[0] = fmaf(f[e / 4].x, __uint_as_float(x[0]), s[0]);
+                        s[1] = fmaf(f[e / 4].y, __uint_as_float(x[1]), s[1]);
+                        s[2] = fmaf(f[e / 4].z, __uint_as_float(x[2]), s[2]);
+                        s[3] = fmaf(f[e / 4].w, __uint_as_float(x[3]), s[3]);
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(tmem_empty_bar(a));
-                mbar_arrive(sc_empty_bar(slot));
-            }
+            if (lane == 0) mbar_arrive(tmem_empty_bar(a));
             if (++a == nbuf) {
                 a = 0;
                 acc_phase ^= 1;
             }
-            if (++slot == kScaleSlots) {
-                slot = 0;
-                sc_phase ^= 1;
-            }
+            if (++slot == kScaleSlots) slot = 0;
         }
     } else {
         mbar_wait(tmem_full_bar(0), 0, ab, 5);
