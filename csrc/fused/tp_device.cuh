@@ -448,13 +448,12 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
             uint4 v[kU];
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                const uint32_t j = j0 + (uint32_t)u * kCopierThreads + (uint32_t)tid;
-                if (j < total) {
-                    const uint32_t b = j / cnt, i = j - b * cnt;
-                    const int      blk = blk_of((int)b);
-                    const char    *src = reinterpret_cast<const char *>(scales ? (const void *)p.sg[blk / mbs] : (const void *)p.xg[blk / mbs]);
-                    v[u] = nvl::ld_nc16(src + (size_t)blk * bytes_per_blk + (first + i) * 16);
-                }
+                // unconditional (past the end the last item again): behind a branch a load would wait for the one before it
+                const uint32_t j = min(j0 + (uint32_t)u * kCopierThreads + (uint32_t)tid, total - 1);
+                const uint32_t b = j / cnt, i = j - b * cnt;
+                const int      blk = blk_of((int)b);
+                const char    *src = reinterpret_cast<const char *>(scales ? (const void *)p.sg[blk / mbs] : (const void *)p.xg[blk / mbs]);
+                v[u] = nvl::ld_nc16(src + (size_t)blk * bytes_per_blk + (first + i) * 16);
             }
 #pragma unroll
             for (int u = 0; u < kU; u++) {
