@@ -12,6 +12,7 @@ import torch
 
 from .. import _capi as K
 from ..api import XcclError, dtype_of
+from ._args import array, stream
 
 _pp = C.POINTER(C.c_void_p)
 K.optional("xccl_nvlink_emu_create", C.c_int, C.c_int, C.c_size_t, _pp)
@@ -23,7 +24,7 @@ K.optional("xccl_nvlink_emu_timeout_probe", C.c_int, C.c_void_p, C.c_int, C.POIN
 
 
 def _ptrs(ts: Optional[Sequence[torch.Tensor]], n: int):
-    arr = (C.c_void_p * n)()
+    arr = array(n)
     if ts is not None:
         for i, t in enumerate(ts):
             arr[i] = t.data_ptr() if t is not None else None
@@ -45,10 +46,10 @@ class EmuWorld:
 
     def _run(self, coll, srcs, dsts, count=0, length=0, dt=K.DT_UINT8, out_dt=K.DT_UNSUPPORTED, op=K.OP_SUM,
              root=0, scale=1.0, alg=0, vmeta=None, max_src_bytes=0, es=1, blocks=0) -> None:
-        s = torch.cuda.current_stream().cuda_stream
         st = K.load().xccl_nvlink_emu_collective(self.h, coll, _ptrs(srcs, self.n), _ptrs(dsts, self.n), count,
-                                                 length, dt, out_dt, op, root, scale, alg, _ptrs(vmeta, self.n),
-                                                 max_src_bytes, es, blocks, s)
+                                                 length, dt, out_dt, op, root, scale, alg,
+                                                 None if vmeta is None else _ptrs(vmeta, self.n), max_src_bytes, es, blocks,
+                                                 stream())
         if st != K.OK:
             raise XcclError(st, f"emulated collective {coll}")
 

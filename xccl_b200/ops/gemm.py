@@ -7,15 +7,12 @@ import torch
 
 from .. import _capi as K
 from ..api import XcclError
+from ._args import stream as _stream
 
 K.optional("xccl_gemm_bf16", C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p)
 K.optional("xccl_gemm_swiglu_bf16", C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
            C.c_int, C.c_void_p)
 K.optional("xccl_gemm_last_error", C.c_uint32)
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _check_bf16(*ts: torch.Tensor) -> None:

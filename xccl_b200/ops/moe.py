@@ -8,6 +8,7 @@ import torch
 
 from .. import _capi as K
 from ..api import XcclError
+from ._args import pointers as _ptrs, stream
 
 _pp = C.POINTER(C.c_void_p)
 K.optional("xccl_moe_ws_create", C.c_int, C.POINTER(K.Oob), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _pp)
@@ -19,15 +20,6 @@ K.optional("xccl_moe_ws_cap_rows", C.c_int, C.c_void_p)
 K.optional("xccl_moe_ws_error", C.c_uint32, C.c_void_p)
 
 BUF_RECV, BUF_EXPERT_OUT, BUF_EXPERT_ROWS, BUF_ROW_SOURCE = range(4)
-
-
-def _ptrs(ts: Sequence[torch.Tensor]):
-    arr = (C.c_void_p * len(ts))()
-    for i, t in enumerate(ts):
-        if not t.is_cuda or not t.is_contiguous():
-            raise ValueError("expected contiguous CUDA tensors")
-        arr[i] = t.data_ptr()
-    return arr
 
 
 class _Workspace:
@@ -93,13 +85,12 @@ class MoeWorkspace:
         return _view(self._buf(local, BUF_ROW_SOURCE), (self.cap_rows,), torch.int32, self.device, self._ws)
 
     def dispatch(self, x: Sequence[torch.Tensor], ids: Sequence[torch.Tensor]) -> None:
-        st = K.load().xccl_moe_dispatch(self.h, _ptrs(x), _ptrs(ids), torch.cuda.current_stream().cuda_stream)
+        st = K.load().xccl_moe_dispatch(self.h, _ptrs(x), _ptrs(ids), stream())
         if st != K.OK:
             raise XcclError(st, "xccl_moe_dispatch")
 
     def combine(self, ids: Sequence[torch.Tensor], weights: Sequence[torch.Tensor], out: Sequence[torch.Tensor]) -> None:
-        st = K.load().xccl_moe_combine(self.h, _ptrs(ids), _ptrs(weights), _ptrs(out),
-                                       torch.cuda.current_stream().cuda_stream)
+        st = K.load().xccl_moe_combine(self.h, _ptrs(ids), _ptrs(weights), _ptrs(out), stream())
         if st != K.OK:
             raise XcclError(st, "xccl_moe_combine")
 

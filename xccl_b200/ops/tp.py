@@ -13,6 +13,7 @@ import torch
 
 from .. import _capi as K
 from ..api import XcclError
+from ._args import pointers as _raw_ptrs, stream
 
 _pp = C.POINTER(C.c_void_p)
 K.optional("xccl_tp_ws_create", C.c_int, C.POINTER(K.Oob), C.c_int, C.c_int, C.c_int, C.c_int, _pp)
@@ -34,21 +35,7 @@ K.optional("xccl_tp_gemm_rs_fp8", C.c_int, C.c_void_p, _pp, _pp, _pp, _pp, _pp, 
 
 
 def _ptrs(ts: Sequence[torch.Tensor]):
-    arr = (C.c_void_p * len(ts))()
-    for i, t in enumerate(ts):
-        if t.dtype != torch.bfloat16 or not t.is_contiguous() or not t.is_cuda:
-            raise ValueError("expected contiguous CUDA bf16 tensors")
-        arr[i] = t.data_ptr()
-    return arr
-
-
-def _raw_ptrs(ts: Sequence[torch.Tensor], dtype: torch.dtype):
-    arr = (C.c_void_p * len(ts))()
-    for i, t in enumerate(ts):
-        if t.dtype != dtype or not t.is_contiguous() or not t.is_cuda:
-            raise ValueError(f"expected contiguous CUDA {dtype} tensors")
-        arr[i] = t.data_ptr()
-    return arr
+    return _raw_ptrs(ts, torch.bfloat16)
 
 
 def quantize_rows(x: torch.Tensor, out8: torch.Tensor, scales: torch.Tensor) -> None:
@@ -57,7 +44,7 @@ def quantize_rows(x: torch.Tensor, out8: torch.Tensor, scales: torch.Tensor) -> 
     if x.dtype != torch.bfloat16 or not x.is_contiguous():
         raise ValueError("expected a contiguous bf16 matrix")
     st = K.load().xccl_tp_quantize_rows(x.data_ptr(), rows, Kd, out8.data_ptr(), scales.data_ptr(),
-                                        torch.cuda.current_stream().cuda_stream)
+                                        stream())
     if st != K.OK:
         raise XcclError(st, "xccl_tp_quantize_rows")
 
@@ -109,14 +96,14 @@ class TpWorkspace:
                        out: Sequence[torch.Tensor]) -> None:
         f_local = w_gate[0].shape[0]
         st = K.load().xccl_tp_ag_gemm_swiglu(self.h, _ptrs(w_gate), _ptrs(w_up), _ptrs(out), f_local,
-                                             torch.cuda.current_stream().cuda_stream)
+                                             stream())
         if st != K.OK:
             raise XcclError(st, "xccl_tp_ag_gemm_swiglu")
 
     def gemm_rs(self, h: Sequence[torch.Tensor], w_down: Sequence[torch.Tensor], out: Sequence[torch.Tensor]) -> None:
         f_local = h[0].shape[1]
         st = K.load().xccl_tp_gemm_rs(self.h, _ptrs(h), _ptrs(w_down), _ptrs(out), f_local,
-                                      torch.cuda.current_stream().cuda_stream)
+                                      stream())
         if st != K.OK:
             raise XcclError(st, "xccl_tp_gemm_rs")
 
@@ -169,7 +156,7 @@ class TpWorkspace:
         f8, f32 = torch.float8_e4m3fn, torch.float32
         st = K.load().xccl_tp_ag_gemm_swiglu_fp8(self.h, _raw_ptrs(w_gate8, f8), _raw_ptrs(s_gate, f32), _raw_ptrs(w_up8, f8),
                                                  _raw_ptrs(s_up, f32), _ptrs(out), f_local,
-                                                 torch.cuda.current_stream().cuda_stream)
+                                                 stream())
         if st != K.OK:
             raise XcclError(st, "xccl_tp_ag_gemm_swiglu_fp8")
 
@@ -181,7 +168,7 @@ class TpWorkspace:
         f8, f32 = torch.float8_e4m3fn, torch.float32
         st = K.load().xccl_tp_ag_gemm_swiglu_fp8q(self.h, _raw_ptrs(w_gate8, f8), _raw_ptrs(s_gate, f32), _raw_ptrs(w_up8, f8),
                                                   _raw_ptrs(s_up, f32), _raw_ptrs(out8, f8), _raw_ptrs(out_scales, f32),
-                                                  f_local, torch.cuda.current_stream().cuda_stream)
+                                                  f_local, stream())
         if st != K.OK:
             raise XcclError(st, "xccl_tp_ag_gemm_swiglu_fp8q")
 
@@ -190,7 +177,7 @@ class TpWorkspace:
         f8, f32 = torch.float8_e4m3fn, torch.float32
         st = K.load().xccl_tp_gemm_rs_fp8(self.h, _raw_ptrs(h8, f8), _raw_ptrs(s_h, f32), _raw_ptrs(w_down8, f8),
                                           _raw_ptrs(s_down, f32), _ptrs(out), f_local,
-                                          torch.cuda.current_stream().cuda_stream)
+                                          stream())
         if st != K.OK:
             raise XcclError(st, "xccl_tp_gemm_rs_fp8")
 
