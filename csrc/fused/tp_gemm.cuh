@@ -39,7 +39,7 @@ struct GemmParams {
     int tp_size;          // ranks taking part (1 without communication)
     int rank_base;        // team rank of blockIdx.y == 0
     int n_gemm_ctas;      // CTAs (per rank) that run MMA tiles; the rest copy (allgather mode, copy_mode 0)
-    int copy_mode;        // allgather mode: 0 = whole CTAs set aside for the copy, 1 = two copier warps in every CTA
+    int copy_mode;        // allgather mode: 0 = whole CTAs set aside for the copy, 1 = copier warps in every CTA (bf16 two, fp8 one)
     int group_rows;       // row blocks of tiles walked together before moving along N (0 = chosen from the shape)
     int group_ramp;       // order of the tile walk while input rows are still arriving from the host.
                           // 1: the groups of the local rows are 1, 1, 2, 4, ... row blocks high, so the first wave of

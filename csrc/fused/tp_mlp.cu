@@ -201,7 +201,7 @@ xccl_status_t xccl_tp_ws_create(const xccl_oob_collectives_t *oob, int emu_ranks
     // Copy mode 0 (whole copy CTAs, bulk copies through shared memory): one SM pulls only 16-20 GB/s over NVLink
     // (measured on 8 GPUs: 4 copy CTAs 1.52 ms, 8: 0.92 ms, 16: 0.76 ms for the 8192 x 7168 x 8192 projection whose MMAs
     // take 0.68 ms), so 16 of them are needed to stay ahead of the tile walk, and each costs tensor throughput.
-    // Copy mode 1 (two copier warps in every CTA, plain loads) costs no tensor throughput but moves only about
+    // Copy mode 1 (copier warps in every CTA, plain loads) costs no tensor throughput but moves only about
     // 120 GB/s per GPU however many loads it keeps in flight (8 GPUs: 1.12 ms), enough for two ranks (67 MB in 2.5 ms:
     // 4.16 ms per block step against 4.41 ms with copy CTAs), not for eight.
     w->copy_ctas_auto = w->copy_ctas <= 0;
