@@ -1173,3 +1173,27 @@ def test_tp_mlp_fp8_fused_matches_dequantised_reference(dev, tp, fuse_quant):
     finally:
         mlp.close()
     _loaded_native()
+
+
+def test_silu_is_as_exact_as_a_rounded_division(dev):
+    """silu in 32 bits against 64: what the fast exponential is documented to lose (2 + 1.173 |x| units of 2^-23, of which the
+    quotient keeps the share e^-x / (1 + e^-x)), half a unit for the sum and half for a rounded division (1e-9 for the
+    squares of these). A quotient that is good to two units only lies outside."""
+    import ctypes as C
+    n = 1 << 21
+    g = torch.Generator(device=dev).manual_seed(3)
+    x = torch.cat([torch.randn(n, device=dev, generator=g) * 4, torch.rand(n, device=dev, generator=g) * 200 - 100,
+                   torch.tensor([0.0, -0.0, 1e-30, -1e-30, 16.7, 88.8, -86.99, -87.0, -87.01, -88.7, 3e38], device=dev)])
+    y = torch.empty_like(x)
+    fn = K.load().xccl_tp_silu
+    fn.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]
+    assert fn(x.data_ptr(), y.data_ptr(), x.numel(), torch.cuda.current_stream().cuda_stream) == K.OK
+    xd = x.double()
+    want = xd / (1 + torch.exp(-xd))
+    lost = (2 + 1.173 * xd.abs()) * 2.0 ** -23 * torch.sigmoid(-xd) + 2.0 ** -23 + 1e-9
+    assert bool(((y.double() - want).abs() <= lost * want.abs() + 2.0 ** -149).all())
+    ends = torch.tensor([float("inf"), float("-inf"), float("nan"), -3e38], device=dev)
+    out = torch.empty_like(ends)
+    assert fn(ends.data_ptr(), out.data_ptr(), 4, torch.cuda.current_stream().cuda_stream) == K.OK
+    out = out.tolist()
+    assert out[0] == float("inf") and out[1] != out[1] and out[2] != out[2] and out[3] == 0
