@@ -1197,3 +1197,47 @@ def test_silu_is_as_exact_as_a_rounded_division(dev):
     assert fn(ends.data_ptr(), out.data_ptr(), 4, torch.cuda.current_stream().cuda_stream) == K.OK
     out = out.tolist()
     assert out[0] == float("inf") and out[1] != out[1] and out[2] != out[2] and out[3] == 0
+
+
+@pytest.mark.parametrize("tp,tokens,hidden,ffn", [(2, 2048, 1152, 3840), (2, 2048, 2048, 4096), (4, 2048, 1152, 4608), (4, 2048, 2048, 4096)])
+def test_tp_mlp_fp8_walkers_of_local_and_gathered_tiles(dev, tp, tokens, hidden, ffn):
+    """The fp8 block over emulated ranks with three to four tiles for every walker, local rows first and gathered rows after
+    them: scales that differ strongly from row to row and from K block to K block reach the right tile, and those of gathered
+    rows are read when they have arrived. K in groups of four blocks (16-byte scale loads) and not."""
+    from xccl_b200.models.tp_mlp import TpMlpFp8
+    from xccl_b200.ops import gemm
+    mlp = TpMlpFp8(tokens, hidden, ffn, tp=tp, emulate=True, fuse_quant=False)
+    g = torch.Generator(device=dev).manual_seed(11)
+    # powers of two, one per block of 128
+    steps = lambda n, lo, hi: torch.exp2(torch.randint(lo, hi + 1, (n // 128,), device=dev, generator=g).float()).repeat_interleave(128)
+    try:
+        for r in range(tp):
+            for name, w, q, s in (("gate", mlp.w_gate, mlp.w_gate8, mlp.s_gate), ("up", mlp.w_up, mlp.w_up8, mlp.s_up),
+                                  ("down", mlp.w_down, mlp.w_down8, mlp.s_down)):
+                rows, cols = w[r].shape
+                v = torch.randn(rows, cols, device=dev, generator=g) * 0.02 * steps(rows, -2, 2)[:, None] * steps(cols, -2, 2)
+                w[r].copy_(v)
+                q8, sc = gemm.quantize_weight_128x128(w[r])
+                q[r].copy_(q8)
+                s[r].copy_(sc)
+        deq = lambda q, s, b: gemm.dequantize(q, s, b).double()
+        for it in range(3):
+            x = torch.randn(tokens, hidden, device=dev, generator=g) * steps(hidden, -2, 2)
+            x = (x * torch.exp2(torch.randint(-3, 3, (tokens, 1), device=dev, generator=g).float())).to(torch.bfloat16)
+            y = mlp.forward(list(x.chunk(tp, 0)))
+            mlp.check_error()
+            xq = deq(torch.cat(mlp.x8, 0), torch.cat(mlp.sx, 0), 1)
+            want, lost = torch.zeros(tokens, hidden, dtype=torch.float64, device=dev), 0.0
+            for r in range(tp):
+                gate, up = xq @ deq(mlp.w_gate8[r], mlp.s_gate[r], 128).t(), xq @ deq(mlp.w_up8[r], mlp.s_up[r], 128).t()
+                h = gate / (1 + torch.exp(-gate)) * up
+                # half a unit of bf16 (2^-9), and 32-bit sums: far below 2e-5 of the row's largest gate and up values, of which
+                # silu (slope at most 1.1) passes on both products
+                sums = 2.1 * 2e-5 * gate.abs().amax(-1, keepdim=True) * up.abs().amax(-1, keepdim=True)
+                assert bool(((mlp.h[r].double() - h).abs() <= 2 ** -8 * h.abs() + sums).all())
+                part = deq(mlp.h8[r], mlp.sh[r], 1) @ deq(mlp.w_down8[r], mlp.s_down[r], 128).t()
+                want += part
+                lost = lost + 2 ** -8 * part.abs() + 2e-5 * part.abs().amax(-1, keepdim=True)   # every partial tile travels as bf16
+            assert bool(((torch.cat(y, 0).double() - want).abs() <= lost + 2 ** -8 * want.abs()).all())
+    finally:
+        mlp.close()
