@@ -409,6 +409,26 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
         if (kCopierThreads == 32) __syncwarp();
         else asm volatile("bar.sync 6, %0;" ::"n"(kCopierThreads) : "memory");
     };
+    // The same, and whether no wait of this CTA has run out: one answer for all copiers, who meet again only if they agree.
+    auto sync_all_well = [&]() -> bool {
+        const uint32_t well = *ab.smem == 0;
+        if (kCopierThreads == 32) {
+            __syncwarp();
+            return __all_sync(0xffffffffu, well) != 0;
+        }
+        uint32_t all;
+        asm volatile(
+            "{\n"
+            ".reg .pred p, q;\n"
+            "setp.ne.u32 p, %1, 0;\n"
+            "bar.red.and.pred q, 6, %2, p;\n"
+            "selp.u32 %0, 1, 0, q;\n"
+            "}\n"
+            : "=r"(all)
+            : "r"(well), "n"(kCopierThreads)
+            : "memory");
+        return all != 0;
+    };
     bool ok = true;
 
     if (me == 0) {
@@ -438,9 +458,8 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
             red_release_gpu_add(go, 1u);   // go counts launches: seq
         }
     }
-    if (tid == 0) ok = wait_counter(go, p.seq, false, ab, 0xa);
-    sync_copiers();
-    ok = (*ab.smem == 0);
+    if (tid == 0) wait_counter(go, p.seq, false, ab, 0xa);
+    ok = sync_all_well();
 
     // The remote row blocks in the order the tile walk needs them; this CTA copies packs [lo, hi) of each. All of it is
     // one sequence of items (block, pack) walked in batches of kCopierThreads x kU, whatever block an item belongs to:
@@ -473,8 +492,7 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
                     *reinterpret_cast<uint4 *>(dst + (size_t)blk * bytes_per_blk + (first + i) * 16) = v[u];
                 }
             }
-            sync_copiers();
-            ok = (*ab.smem == 0);
+            ok = sync_all_well();
             if (announce_blocks && tid == 0) {
                 const uint32_t stored = min(j0 + (uint32_t)(kCopierThreads * kU), total);
                 if ((uint32_t)(announced + 1) * cnt <= stored) {
