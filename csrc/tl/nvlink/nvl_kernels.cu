@@ -19,6 +19,7 @@
 // is produced, so gradient averaging and fp32->bf16 casting cost no extra pass over memory.
 // Baseline these replace: the reference's NCCL team, src/team_lib/nccl/xccl_nccl_collective.c:40-231.
 #include <algorithm>
+#include <type_traits>
 
 #include "../../cuda/cuda_common.h"
 #include "../../cuda/dev_types.cuh"
@@ -178,14 +179,45 @@ __device__ __forceinline__ void stream_packs(size_t lo, size_t hi, LoadFn ld, St
     for (; i < hi; i += bd) st(i, ld(i));
 }
 
-// The same for a kernel whose blocks take turns along [lo, hi), tile by tile (zero-copy kernels on large buffers; the staged
-// ones need block b to stay in its own piece). Blocks that each walk a range of their own spread the DRAM's pages: 134 MB read
-// and 134 MB written by 296 blocks 53.5 us, taking turns 49.5.
-template <int U, typename LoadFn, typename StoreFn>
-__device__ __forceinline__ void stream_tiles(size_t lo, size_t hi, LoadFn ld, StoreFn st)
+// Packs of a tile where the blocks of a kernel take turns along n packs (zero-copy kernels on large buffers; the staged ones need
+// block b to stay in its own piece). At most `most`, and as few turns as that allows, shared evenly: a short piece is one turn of
+// all blocks (fixed tiles of 32 KiB left 296 blocks only 24 turns in a segment of 768 KiB), a long one ends with all of them
+// (128 tiles for 37 blocks are four turns for some and three for the rest; 256 smaller ones seven for all but three). On the host:
+// its divisions, once per segment, cost the kernel 2 us with eight ranks.
+inline size_t turn_tile(size_t n, size_t blocks, size_t most)
 {
-    const size_t tile = (size_t)U * blockDim.x;
-    for (size_t t = lo + blockIdx.x * tile; t < hi; t += gridDim.x * tile) stream_packs<U>(t, min(t + tile, hi), ld, st);
+    const size_t per = (n + blocks - 1) / blocks, turns = (per + most - 1) / most;
+    return turns == 0 ? 32 : ((per + turns - 1) / turns + 31) / 32 * 32;
+}
+
+// [lo, hi) with blocks taking turns. Blocks that each walk a range of their own spread the DRAM's pages: 134 MB read and 134 MB
+// written by 296 blocks 53.5 us, taking turns 49.5. All loads of a tile are in flight before its first store, also where it is
+// not a whole U x blockDim.
+template <int U, typename LoadFn, typename StoreFn>
+__device__ __forceinline__ void stream_tiles(size_t lo, size_t hi, size_t tile, LoadFn ld, StoreFn st)
+{
+    const size_t bd = blockDim.x;
+    auto steps = [&](size_t t, size_t end, auto n) {
+        constexpr int N = decltype(n)::value;
+        const size_t  i = t + threadIdx.x;
+        uint4         v[N];
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            if (u < N - 1 || i + u * bd < end) v[u] = ld(i + u * bd);
+        }
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            if (u < N - 1 || i + u * bd < end) st(i + u * bd, v[u]);
+        }
+    };
+    static_assert(U == 4, "steps of a tile");
+    for (size_t t = lo + blockIdx.x * tile; t < hi; t += gridDim.x * tile) {
+        const size_t end = min(t + tile, hi), len = end - t;
+        if (len > 3 * bd) steps(t, end, std::integral_constant<int, 4>{});
+        else if (len > 2 * bd) steps(t, end, std::integral_constant<int, 3>{});
+        else if (len > bd) steps(t, end, std::integral_constant<int, 2>{});
+        else steps(t, end, std::integral_constant<int, 1>{});
+    }
 }
 
 // Reduces pack i of n source arrays (src_of(q) + i * 16) and hands the accumulators to out(i, acc).
@@ -256,9 +288,8 @@ __device__ __forceinline__ void reduce_packs(SrcFn src_of, int n, size_t lo, siz
 
 // Blocks taking turns, as in stream_tiles.
 template <typename T, bool kSum, typename SrcFn, typename OutFn>
-__device__ __forceinline__ void reduce_tiles(SrcFn src_of, int n, size_t lo, size_t hi, int op, OutFn out)
+__device__ __forceinline__ void reduce_tiles(SrcFn src_of, int n, size_t lo, size_t hi, size_t tile, int op, OutFn out)
 {
-    const size_t tile = 2 * (size_t)blockDim.x;
     for (size_t t = lo + blockIdx.x * tile; t < hi; t += gridDim.x * tile) reduce_packs<T, kSum, 2>(src_of, n, t, min(t + tile, hi), op, out);
 }
 
@@ -748,7 +779,7 @@ __global__ void __launch_bounds__(512) direct_reduce_kernel(World w, Call c)
             O          *dst = (O *)c.dst[s.local];
             const size_t seg_bytes = c.count * sizeof(T);
             reduce_tiles<T, kSum>([&](int q) { return (const char *)c.peer_src[q] + (size_t)s.rank * seg_bytes; }, w.size, 0, npacks,
-                                  c.op, [&](size_t i, A(&acc)[E]) {
+                                  c.tile, c.op, [&](size_t i, A(&acc)[E]) {
 #pragma unroll
                                       for (int e = 0; e < E; e++) acc[e] = dev::scaled(acc[e], c.scale, c.do_scale != 0);
                                       store_out<O, E>(dst, i, c.count, true, acc);
@@ -756,7 +787,7 @@ __global__ void __launch_bounds__(512) direct_reduce_kernel(World w, Call c)
         } else {
             const size_t per = (npacks + w.size - 1) / w.size;
             const size_t lo  = min((size_t)s.rank * per, npacks), hi = min(lo + per, npacks);
-            reduce_tiles<T, kSum>([&](int q) { return (const char *)c.peer_src[q]; }, w.size, lo, hi, c.op,
+            reduce_tiles<T, kSum>([&](int q) { return (const char *)c.peer_src[q]; }, w.size, lo, hi, c.tile, c.op,
                                   [&](size_t i, A(&acc)[E]) {
 #pragma unroll
                                       for (int e = 0; e < E; e++) acc[e] = dev::scaled(acc[e], c.scale, c.do_scale != 0);
@@ -780,16 +811,17 @@ template <int KIND> __global__ void __launch_bounds__(512) direct_mover_kernel(W
     const size_t npacks    = seg_bytes / 16;
     block_barrier(w, s);
     if (!s.failed) {
-        // every rank starts with itself, so that the peers' links share the load; emulated ranks read one memory, and in an
-        // allgather all of them the same source at a time, from L2 after the first (8 x 16 MB: 394 us, now 242)
-        const int first = KIND == MV_ALLGATHER && w.n_local > 1 ? 0 : s.rank;
+        // Every rank starts with itself, so that the peers' links share the load. Emulated ranks read one memory: in an allgather
+        // whose sources do not stay in L2 beside the output, all of them read the same source at a time, from L2 after the first
+        // (8 x 16 MB: 394 us, so 242; 8 x 3 MB 78 and 73; but 8 x 1 MB 46.9 and 48.0, 8 x 256 KB 39.7 and 41.8).
+        const int first = KIND == MV_ALLGATHER && w.n_local > 1 && c.len > ((size_t)16 << 20) ? 0 : s.rank;
         for (int q = 0; q < w.size; q++) {
             const int   p    = (first + q) % w.size;
             const char *from = (const char *)c.peer_src[p] + ((KIND == MV_ALLTOALL) ? (size_t)s.rank * seg_bytes : 0);
             char       *out  = (char *)dst + (size_t)p * seg_bytes;
             if (from == out) continue;  // in-place allgather: my own segment is where it belongs
             stream_tiles<4>(
-                0, npacks, [&](size_t i) { return ld_nc16(from + i * 16); }, [&](size_t i, uint4 v) { st_16(out + i * 16, v); });
+                0, npacks, c.tile, [&](size_t i) { return ld_nc16(from + i * 16); }, [&](size_t i, uint4 v) { st_16(out + i * 16, v); });
         }
         block_barrier(w, s);
     }
@@ -1047,7 +1079,9 @@ xccl_status_t direct_reduce_typed(const World &w, const Call &c, const LaunchCfg
     auto          k      = sum ? direct_reduce_kernel<T, O, true, kScatter> : direct_reduce_kernel<T, O, false, kScatter>;
     const size_t  mine   = kScatter ? npacks : (npacks + w.size - 1) / w.size;
     int           blocks = pick_blocks(k, w, cfg, mine, 2);
-    return launch(k, dim3((unsigned)blocks, (unsigned)w.n_local), dim3((unsigned)cfg.threads), cfg.cooperative, stream, w, c);
+    Call          call   = c;
+    call.tile = turn_tile(mine, (size_t)blocks, (E <= 8 && w.size <= 4 ? 2 : 1) * (size_t)cfg.threads);   // packs a thread has in flight (reduce_packs)
+    return launch(k, dim3((unsigned)blocks, (unsigned)w.n_local), dim3((unsigned)cfg.threads), cfg.cooperative, stream, w, call);
 }
 template <bool kScatter>
 xccl_status_t direct_reduce_dispatch(const World &w, const Call &c, xccl_dt_t dt, xccl_dt_t out_dt, const LaunchCfg &cfg,
@@ -1071,15 +1105,14 @@ xccl_status_t launch_direct(const World &w, const Call &c, int coll, xccl_dt_t d
     switch (coll) {
     case XCCL_ALLREDUCE: return direct_reduce_dispatch<false>(w, c, dt, out_dt, cfg, stream);
     case XCCL_REDUCE_SCATTER: return direct_reduce_dispatch<true>(w, c, dt, out_dt, cfg, stream);
-    case XCCL_ALLGATHER: {
-        auto k      = direct_mover_kernel<MV_ALLGATHER>;
-        int  blocks = pick_blocks(k, w, cfg, c.len / 16, 4);
-        return launch(k, dim3((unsigned)blocks, (unsigned)w.n_local), dim3((unsigned)cfg.threads), cfg.cooperative, stream, w, c);
-    }
+    case XCCL_ALLGATHER:
     case XCCL_ALLTOALL: {
-        auto k      = direct_mover_kernel<MV_ALLTOALL>;
-        int  blocks = pick_blocks(k, w, cfg, c.len * (size_t)w.size / 16, 4);
-        return launch(k, dim3((unsigned)blocks, (unsigned)w.n_local), dim3((unsigned)cfg.threads), cfg.cooperative, stream, w, c);
+        auto         k      = coll == XCCL_ALLGATHER ? direct_mover_kernel<MV_ALLGATHER> : direct_mover_kernel<MV_ALLTOALL>;
+        const size_t seg    = (coll == XCCL_ALLGATHER ? c.len / w.size : c.len) / 16;
+        int          blocks = pick_blocks(k, w, cfg, seg * (size_t)w.size, 4);
+        Call         call   = c;
+        call.tile = turn_tile(seg, (size_t)blocks, 4 * (size_t)cfg.threads);   // every segment anew, from block 0
+        return launch(k, dim3((unsigned)blocks, (unsigned)w.n_local), dim3((unsigned)cfg.threads), cfg.cooperative, stream, w, call);
     }
     default: return XCCL_ERR_UNSUPPORTED;
     }
@@ -1235,6 +1268,9 @@ extern "C" int xccl_nvlink_debug_bounds_ranges(unsigned long long *lo, unsigned 
     return -1;
 #endif
 }
+
+// Host-side view of the turns (tests): packs of a tile where `blocks` blocks take turns along n packs.
+extern "C" size_t xccl_nvlink_turn_tile(size_t n, size_t blocks, size_t most) { return xccl::nvl::turn_tile(n, blocks, most); }
 
 // Record of the bounds-checking build: out[0] = accesses that were refused since the last call, out[1] = the first
 // refused address, out[2] = its kind (1 store, 2 load, 3 multicast store, 4 multicast load), out[3] = (rank << 32) |

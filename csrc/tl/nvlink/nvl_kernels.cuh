@@ -31,6 +31,8 @@ struct Call {
     // allocation they live in (same offset on every rank), by LOCAL rank.
     const void     *mc_src[kMaxRanks];
     void           *mc_dst[kMaxRanks];
+    // Direct algorithms: packs of a tile, where the blocks take turns (set by the launch).
+    size_t          tile;
 };
 
 enum Alg { ALG_AUTO = 0, ALG_ONE_SHOT = 1, ALG_TWO_SHOT = 2, ALG_NVLS = 3, ALG_DIRECT = 4, ALG_SYMMETRIC = 5 };

@@ -1241,3 +1241,29 @@ def test_tp_mlp_fp8_walkers_of_local_and_gathered_tiles(dev, tp, tokens, hidden,
             assert bool(((torch.cat(y, 0).double() - want).abs() <= lost + 2 ** -8 * want.abs()).all())
     finally:
         mlp.close()
+
+
+@pytest.mark.parametrize("n,blocks", [(2, 0), (4, 3), (8, 0), (8, 18)])
+@pytest.mark.parametrize("packs", [1, 31, 513, 2047, 2049, 18 * 2048 + 33, 40000])
+def test_emu_direct_turns_of_the_blocks(dev, n, blocks, packs):
+    """Zero-copy collectives whose segments give a block a part of one tile, a whole one and several: every pack arrives, and
+    nothing behind a destination is written."""
+    from xccl_b200.ops.emu import EmuWorld
+    w = EmuWorld(n, 8 << 20)
+    D, per = K.NVLINK_ALG_DIRECT, packs * 4          # fp32 values of a segment
+    tail = lambda size: [torch.full((size + 64,), -7.0, device=dev) for _ in range(n)]
+    try:
+        src = _ints(n, per * n, torch.float32, dev, seed=packs)
+        run = lambda op, ins, size, **kw: (lambda full: (getattr(w, op)(ins, [f[:size] for f in full], alg=D, **kw), full)[1])(tail(size))
+        total = torch.stack(src).sum(0)
+        want = {"allreduce": [total] * n, "reduce_scatter": list(total.chunk(n)),
+                "allgather": [torch.cat([s[:per] for s in src])] * n,
+                "alltoall": [torch.cat([s[r * per:(r + 1) * per] for s in src]) for r in range(n)]}
+        for op, expected in want.items():
+            ins = [s[:per] for s in src] if op == "allgather" else src
+            kw = {"blocks": blocks} if op == "allreduce" else {}
+            for got, e in zip(run(op, ins, e_size := expected[0].numel(), **kw), expected):
+                assert torch.equal(got[:e_size], e), op
+                assert bool((got[e_size:] == -7).all()), op
+    finally:
+        w.close()
