@@ -94,13 +94,15 @@ namespace {
 
 // Whether a collective for which no algorithm was named runs zero-copy on the user buffers (they are all on this device).
 // The staged kernels pass every byte through the workspaces, which costs little while that traffic stays in L2 and
-// doubles the DRAM traffic beyond it; the zero-copy kernels have one barrier more. Measured on one B200 per call,
-// staged / zero-copy in us, by the bytes of all ranks together: allreduce fp32 8 ranks 2 MB 30.7 / 34.2, 8 MB 47.3 /
-// 34.3, 128 MB 151.5 / 83.2, 2 ranks 8 MB 30.2 / 36.6, 16 MB (bf16) 45.4 / 34.5; reduce-scatter 8 ranks 8 MB 30.6 / 31.6, 32 MB
-// 46.9 / 39.6, 128 MB 104 / 59.5; allgather (output) 8 ranks 64 MB 45.5 / 52.4, 256 MB 120.9 / 105.6; alltoall 8 ranks 16 MB 35.4 /
-// 42.3, 128 MB 135.2 / 82.8. Around the limits: reduce-scatter fp32 4 ranks 20 MB 32.3 / 37.1, 28 MB 37.3 / 38.3, 36
-// MB 42.8 / 39.2, 8 ranks 20 MB 36.3 / 35.2, bf16 4 ranks 16 MB 35.3 / 31.8; allgather 4 ranks 100 MB 60.8 / 61.1, 128 MB 76.4 / 70.1, 6 ranks 112 MB 58.2 / 61.6, 8 ranks 144 MB 64.9 / 74.6, 192 MB
-// 95.2 / 87.7; alltoall 4 ranks 32 MB 46.6 / 47.8, 8 ranks 36 MB 45.9 / 49.6, 40 MB 53.2 / 55.0, 48 MB 67.1 / 59.0.
+// doubles the DRAM traffic beyond it; the zero-copy kernels have one barrier more. Measured on one B200 per call (warm buffers),
+// staged / zero-copy in us, by the bytes of all ranks together, on both sides of the limits: allreduce fp32 8 ranks 6 MB 34.2 / 29.8, 10 MB
+// 37.5 / 29.8, 4 ranks 6 MB 32.3 / 27.2, 10 MB 34.4 / 28.7, 2 ranks 14 MB 34.4 / 29.0, 20 MB 38.5 / 30.7; reduce-scatter fp32 2 ranks 28 MB
+// 33.6 / 28.6, 36 MB 43.7 / 29.3, 4 ranks 28 MB 35.8 / 27.7, 36 MB 43.7 / 28.0, 8 ranks 12 MB 29.3 / 28.1, 20 MB 33.1 / 28.9, bf16 4 ranks 12 MB
+// 28.1 / 27.1, 20 MB 32.5 / 28.0; allgather 2 ranks 90 MB 69.6 / 52.6, 112 MB 81.8 / 57.5, 4 ranks 90 MB 56.5 / 51.6, 112 MB 63.7 / 56.8, 6 ranks
+// 112 MB 59.2 / 59.6, 128 MB 70.3 / 60.5, 8 ranks 144 MB 65.7 / 60.8, 192 MB 97.0 / 70.6; alltoall 4 ranks 28 MB 41.8 / 36.0, 36 MB 53.6 / 37.5, 8 ranks
+// 44 MB 58.7 / 41.4, 64 MB 86.3 / 48.7. Zero-copy is not slower anywhere above its limit. Most limits were drawn for zero-copy kernels
+// that were slower and lie above the crossover: it is at or below 2 MB for allreduce, at 12 MB for reduce-scatter, 24 to 28 MB for alltoall,
+// and for allgather at 48 MB (2 ranks), 64 MB (4), 80 MB (6) and 96 MB (8).
 bool direct_pays(const World &w, const Call &c, int coll, xccl_dt_t dt, xccl_dt_t out_dt)
 {
     if (out_dt == XCCL_DT_UNSUPPORTED || out_dt == XCCL_DT_LAST_PREDEFINED) out_dt = dt;
