@@ -550,12 +550,15 @@ bool skinny_plan(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan
 // Rows beyond one MMA, in blocks of up to 128: where the tiles of the large kernel (256 x 256, in bf16 narrower ones too) leave
 // most of the chip idle, small tiles whose K is shared by a cluster fill it, although each block of rows reads the weights
 // again (from L2). fp8: as long as every CTA has an SM to itself (the large kernel's fp8 tiles are all 256 columns wide), with
-// SwiGLU only where CTAs share K. bf16: where at least three CTAs share 24 K blocks and more; with fewer it is level or behind,
-// and SwiGLU stays with the large kernel. Large / few-rows kernel, 140 products each of 129 to 1536 rows, N and K from 256 to
-// 8192, L2 flushed: fp8 within the rule 1.50 times faster on average, 1.14 the least (outside 0.6 to 1.0), bf16 1.30 and 0.95
-// (outside 0.91 on average), bf16 SwiGLU 0.89 where the CTAs fit the SMs. fp8 212 x 768 x 7808 54.3 / 20.5 us, 502 x 1664 x 5376
-// 37.9 / 22.5, 8192 x 256 x 512 17.3 / 12.3; bf16 143 x 2928 x 7728 39.9 / 28.7, 370 x 304 x 5216 27.5 / 18.5. fp8 block step (SwiGLU and
-// down projection) 256 rows, 1152, 4352 64.5 / 44.0, 512 rows, 5376, 2944 76.8 (97.2 with unshared SwiGLU tiles).
+// SwiGLU only where CTAs share K. bf16: where at least three CTAs share more than 32 K blocks (with fewer 0.95 to 1.04 of the
+// large kernel's time) and the CTAs are nine tenths of the SMs at most: clusters do not fill every SM, so with more of them some
+// SMs run two and the rest waits for those (135 to 225 CTAs: 0.80 to 1.28 of the large kernel's time, 1.00 on average). SwiGLU in
+// bf16 stays with the large kernel (0.89 of its speed). Operands in DRAM, launches back to back, 83 drawn bf16 products within the
+// rule: 0.81 of the time on average, 1.00 the worst; 110 fp8 products and blocks 0.76 on average, 1.00 the worst. Large / few-rows
+// kernel in us: bf16 206 x 576 x 7160 33.5 / 18.8, 370 x 1280 x 7032 32.9 / 23.0, 1654 x 336 x 3016 18.6 / 18.6, outside 480 x 1528 x 1672
+// 14.4 / 18.5 and 590 x 1816 x 8072 41.1 / 46.2. L2 flushed: fp8 212 x 768 x 7808 54.3 / 20.5, 502 x 1664 x 5376 37.9 / 22.5, 8192 x 256 x 512
+// 17.3 / 12.3; fp8 block step (SwiGLU and down projection) 256 rows, 1152, 4352 64.5 / 44.0, 512 rows, 5376, 2944 76.8 (97.2 with
+// unshared SwiGLU tiles).
 bool skinny_plan_rows(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
 {
     if (M <= kSkinnyMaxM) return skinny_plan(M, N, K, fp8, swiglu, sms, out);
@@ -563,7 +566,8 @@ bool skinny_plan_rows(int M, int N, int K, bool fp8, bool swiglu, int sms, Skinn
     if ((swiglu && !fp8) || blocks > sms) return false;
     SkinnyPlan q{};
     if (!plan_blocks((M - 1) / blocks + 1, blocks, N, K, fp8, swiglu, sms, &q)) return false;
-    if (fp8 ? q.blocks * q.tiles * q.splits > sms || (swiglu && q.splits < 2) : q.splits < 3 || q.kblocks < 24) return false;
+    const int ctas = q.blocks * q.tiles * q.splits;
+    if (fp8 ? ctas > sms || (swiglu && q.splits < 2) : q.splits < 3 || q.kblocks <= 32 || ctas * 10 > sms * 9) return false;
     *out = q;
     return true;
 }

@@ -110,3 +110,16 @@ def test_blocks_of_rows_cover_the_rows_and_keep_to_the_rule(fp8, swiglu):
     assert taken > 20
     assert _plan_rows(300, 1024, 8192, False, True) is None      # bf16 SwiGLU stays with the large kernel
     assert _plan_rows(1 << 30, 128, 128, True, False) is None
+
+
+@pytest.mark.parametrize("M,N,K_,taken", [
+    # large / few-rows kernel in us: 14.4 / 18.5, 21.4 / 26.7, 24.7 / 30.0, 34.9 / 41.6, 20.7 / 24.6, 13.9 / 14.4 (25 K blocks)
+    (480, 1528, 1672, False), (379, 2048, 3480, False), (1006, 736, 4664, False), (1585, 520, 7176, False), (232, 2992, 3240, False),
+    (1145, 288, 1592, False),
+    # 33.5 / 18.8, 32.9 / 23.0, 26.7 / 22.5, 18.6 / 18.6
+    (206, 576, 7160, True), (370, 1280, 7032, True), (480, 1328, 4984, True), (1654, 336, 3016, True)])
+def test_blocks_of_rows_only_where_no_measured_product_is_slower(M, N, K_, taken):
+    p = _plan_rows(M, N, K_, False, False)
+    assert (p is not None) == taken
+    if taken:
+        assert p["blocks"] * p["tiles"] * p["splits"] <= 133 and p["kblocks"] > 32
