@@ -139,6 +139,8 @@ xccl_status_t launch_gemm_fp8(const GemmParams &p, const GemmLaunch &l, cudaStre
 // Tuning options of the fused kernels: the option table "TP_" of the library's configuration system, read once from
 // the environment (XCCL_TP_<NAME>) like every other option table and listed by xccl_tp_config_print().
 const OptTable &tp_options();
+// Whether the user asks for tiles of a certain kind (a width, single CTAs): products that could run elsewhere then use them.
+bool tiles_asked_for(bool fp8);
 
 size_t gemm_smem_bytes();
 uint32_t *error_word();  // per-device error word shared by the GEMM kernels

@@ -572,6 +572,12 @@ bool skinny_plan_rows(int M, int N, int K, bool fp8, bool swiglu, int sms, Skinn
     return true;
 }
 
+// Whether a product runs here: the rule above, unless it is one for tiles and the user asks for a kind of them.
+static bool takes(int M, int N, int K, bool fp8, bool swiglu, int sms, SkinnyPlan *out)
+{
+    return (M <= kSkinnyMaxM || !tiles_asked_for(fp8)) && skinny_plan_rows(M, N, K, fp8, swiglu, sms, out);
+}
+
 bool try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st)
 {
     // what the large kernels refuse is left to them to refuse
@@ -579,7 +585,7 @@ bool try_skinny(const SkinnyArgs &a, cudaStream_t stream, xccl_status_t *st)
     int        dev = 0, sms = 0;
     SkinnyPlan plan;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-    if (!skinny_plan_rows(a.M, a.N, a.K, a.fp8, a.swiglu, sms, &plan)) return false;
+    if (!takes(a.M, a.N, a.K, a.fp8, a.swiglu, sms, &plan)) return false;
     *st = launch_skinny(a, plan, stream);
     if (*st == XCCL_OK) return true;
     (void)cudaGetLastError();   // refused: the large kernel serves the call, or says why not
@@ -647,4 +653,10 @@ extern "C" int xccl_tp_skinny_plan(int M, int N, int K, int fp8, int swiglu, int
 extern "C" int xccl_tp_skinny_plan_rows(int M, int N, int K, int fp8, int swiglu, int sms, int *out)
 {
     return skinny_plan_out(true, M, N, K, fp8 != 0, swiglu != 0, sms, out);
+}
+// Whether such a product runs in this kernel under the options of this process.
+extern "C" int xccl_tp_skinny_takes(int M, int N, int K, int fp8, int swiglu, int sms)
+{
+    xccl::tp::SkinnyPlan q;
+    return xccl::tp::takes(M, N, K, fp8 != 0, swiglu != 0, sms, &q) ? 1 : 0;
 }

@@ -123,3 +123,19 @@ def test_blocks_of_rows_only_where_no_measured_product_is_slower(M, N, K_, taken
     assert (p is not None) == taken
     if taken:
         assert p["blocks"] * p["tiles"] * p["splits"] <= 133 and p["kblocks"] > 32
+
+
+@pytest.mark.parametrize("env,bf16,fp8", [({}, 1, 1), ({"XCCL_TP_GEMM_BN": "64"}, 0, 1), ({"XCCL_TP_GEMM_PAIR": "n"}, 0, 0)])
+def test_tiles_that_are_asked_for_serve_more_than_one_block_of_rows(env, bf16, fp8):
+    """A forced tile width or single CTAs: products of more than 128 rows run in the kernel with these tiles, as its options say
+    (they are read once per process); up to 128 rows are the few-rows kernel's in any case."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    script = ("from xccl_b200 import _capi as K\nf = K.load().xccl_tp_skinny_takes\n"
+              "print(f(640, 232, 4104, 0, 0, 148), f(256, 512, 1536, 1, 0, 148), f(100, 512, 1536, 0, 0, 148), f(100, 512, 1536, 1, 0, 148))")
+    full = {k: v for k, v in os.environ.items() if not k.startswith("XCCL_TP_")}
+    full.update(env, PYTHONPATH=str(Path(__file__).resolve().parent.parent))
+    r = subprocess.run([sys.executable, "-c", script], env=full, capture_output=True, text=True, timeout=120)
+    assert r.stdout.split() == [str(bf16), str(fp8), "1", "1"], r.stdout + r.stderr[-2000:]
