@@ -1267,3 +1267,29 @@ def test_emu_direct_turns_of_the_blocks(dev, n, blocks, packs):
                 assert bool((got[e_size:] == -7).all()), op
     finally:
         w.close()
+
+
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("M,N,K_", [(4096, 4096, 1024), (4096, 4096, 1152), (4000, 4224, 1280), (4096, 4096, 1408), (4096, 6144, 128), (3968, 4096, 2048)])
+def test_gemm_fp8_blockscaled_many_tiles_per_walker(dev, M, N, K_, off):
+    """Three to four tiles for every CTA pair of the large kernel: the scale ring, its phases and the scales loaded ahead go over
+    from tile to tile, for every remainder of the K blocks by four and for scales that do not start on 16 bytes. Scales differ by
+    powers of two from row to row and from K block to K block, so one that is a block off shows."""
+    from xccl_b200.ops import gemm
+    assert K.load().xccl_tp_skinny_plan_rows(M, N, K_, 1, 0, 148, (C.c_int * 11)()) == 0     # the large kernel's
+    g = torch.Generator(device=dev).manual_seed(M + N + K_)
+    steps = lambda n: torch.exp2(torch.randint(-3, 4, (n // 128,), device=dev, generator=g).float()).repeat_interleave(128)
+    a = torch.randn(M, K_, device=dev, generator=g) * torch.exp2(torch.randint(-3, 4, (M, 1), device=dev, generator=g).float()) * steps(K_)
+    b = torch.randn(N, K_, device=dev, generator=g) * 0.05 * steps(N)[:, None] * steps(K_)
+    a8, sa = gemm.quantize_act_1x128(a)
+    b8, sb = gemm.quantize_weight_128x128(b)
+    moved = torch.full((sa.numel() + 8,), float("nan"), device=dev)[off:off + sa.numel()].view_as(sa)
+    moved.copy_(sa)
+    guard = torch.full((M + 2, N), 7.0, device=dev, dtype=torch.bfloat16)
+    for _ in range(2):
+        gemm.gemm_fp8_blockscaled(a8, moved, b8, sb, guard[1:M + 1])
+    assert gemm.last_error() == 0
+    want = gemm.dequantize(a8, sa, 1).double() @ gemm.dequantize(b8, sb, 128).double().t()
+    # half a unit in the last place of bf16 (2^-9), and 32-bit sums of K products far below the largest value of the row
+    assert bool(((guard[1:M + 1].double() - want).abs() <= 2 ** -8 * want.abs() + 2e-5 * want.abs().amax(-1, keepdim=True)).all())
+    assert bool((guard[0] == 7).all()) and bool((guard[M + 1] == 7).all())
