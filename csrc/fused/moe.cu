@@ -457,8 +457,10 @@ template <bool kAlone> __global__ void __launch_bounds__(1024, 1) moe_combine_ke
     }
     // a warp adds up seg_packs packs of one token: lane k holds routing entry k, the warp shares the rows' addresses, and all
     // (up to eight) expert rows of a pack are in flight at once. 4096 x 7168, top 8 (530 MB): 244 us with a warp per whole
-    // token and a branch per load, which made the eight loads wait for one another. The entries of a warp's next piece are
-    // loaded beside the rows of this one, and one rank alone reads without system scope: 104 us, now 97.
+    // token and a branch per load, which made the eight loads wait for one another. One rank alone loads the entries of a warp's
+    // next piece beside the rows of this one and reads without system scope and past L1: 104 us, now 97 (the last costs where the
+    // same rows are read from L2 again and again, 512 x 4096 9.6 and 12.6 us, and nothing behind the kernel that writes them). With
+    // several ranks the early entries only spill: 2048 x 4096, top 4, two ranks 43.6 us, so 45.2, 1024 x 2048, top 10, 27.3 and 29.2.
     const int    lane = threadIdx.x % 32;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32, nwarps = (size_t)gridDim.x * blockDim.x / 32;
     const int    packs = p.H * 2 / 16, nseg = (packs + p.seg_packs - 1) / p.seg_packs;
@@ -479,17 +481,18 @@ template <bool kAlone> __global__ void __launch_bounds__(1024, 1) moe_combine_ke
     int      e_next = -1;
     float    g_next = 0.0f;
     uint32_t r_next = 0;
-    if (warp < items) entry(warp / nseg, 0, e_next, g_next, r_next);
+    if (kAlone && warp < items) entry(warp / nseg, 0, e_next, g_next, r_next);
     for (size_t it = warp; it < items && failed == 0; it += nwarps) {
         const size_t t  = it / nseg;
         const int    lo = (int)(it % nseg) * p.seg_packs, hi = min(lo + p.seg_packs, packs);
         // (with more than eight entries the running sum passes through bf16 between groups)
         for (int kb = 0; kb < p.K; kb += 8) {
+            if (!kAlone) entry(t, kb, e_next, g_next, r_next);
             const bool     on     = e_next >= 0 && e_next < p.E;
             const float    my_g   = on ? g_next : 0.0f;
             const unsigned long long my_row = on ? (unsigned long long)(p.yout[kAlone ? 0 : e_next / EL] + (size_t)r_next * p.H) : 0ull;
-            if (kb + 8 < p.K) entry(t, kb + 8, e_next, g_next, r_next);
-            else if (it + nwarps < items) entry((it + nwarps) / nseg, 0, e_next, g_next, r_next);
+            if (kAlone && kb + 8 < p.K) entry(t, kb + 8, e_next, g_next, r_next);
+            else if (kAlone && it + nwarps < items) entry((it + nwarps) / nseg, 0, e_next, g_next, r_next);
             const uint4 *rows[8];
             float        gs[8];
 #pragma unroll
