@@ -1,10 +1,11 @@
 // MoE expert dispatch / combine fused with the all-to-all (extension; the reference only has
 // alltoallv call sites: src/team_lib/nccl/xccl_nccl_collective.c:125-163).
 //
-// dispatch (ONE kernel; one rank alone has its own, without the exchange): count tokens per expert, exchange the counts with every rank through
-//   peer memory, turn them into receive offsets, and copy every routed token row straight into its
-//   slot of the destination rank's receive buffer - rows arrive grouped by (local expert, source
-//   rank), ready for a grouped GEMM. No host round trip, no intermediate permuted copy.
+// dispatch (ONE kernel; one rank alone has its own, without the exchange): count tokens per expert,
+//   exchange the counts with every rank through peer memory, turn them into receive offsets, and
+//   copy every routed token row straight into its slot of the destination rank's receive buffer -
+//   rows arrive grouped by (local expert, source rank), ready for a grouped GEMM. No host round
+//   trip, no intermediate permuted copy.
 // combine (ONE kernel): every token pulls its top-k expert outputs from the owners' buffers and
 //   adds them up with its gate weights in fp32.
 // Ranks are real (one process per GPU) or emulated (blockIdx.y = rank in one cooperative launch).

@@ -27,13 +27,12 @@ constexpr uint32_t kSmemBytes  = kStages * kStageBytes + kEpiBytes + 256 + 1024;
 constexpr int      kStagesPair = 6;
 static_assert(kStagesPair * (kABytes + kBBytes / 2) == kStages * kStageBytes, "both modes share one shared-memory layout");
 
-// fp8: registers of a thread of the first four warps (loads, MMAs, copiers) and of the eight promotion warps, whose 128 running
-// sums spill with the 168 that twelve warps get alike.
 // fp8: products of the two scales of K blocks ahead, [slot][weight block][row].
 constexpr int      kScaleRing = 4;
 constexpr uint32_t kScaleRingBytes = 2 * kBM * 4;
-// fp8: registers of a thread of the first four warps (loads, MMAs, copier, scales) and of the eight promotion warps, whose 128
-// running sums and 32 values on their way spill with the 168 that twelve warps get alike.
+// fp8: registers of a thread of the first four warps (loads, MMAs, copier, scales) and of the eight promotion warps, which hold 128
+// running sums and 32 values on their way; twelve warps alike would get 168. Some values still spill (bytes stored / loaded per
+// thread: CTA pairs 100 / 256, single CTAs 144 / 212).
 constexpr int      kRegsOthers = 104, kRegsPromotion = 200;
 
 struct Tile {

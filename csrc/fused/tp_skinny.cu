@@ -8,10 +8,10 @@
 // of weight loads in flight. Measured on one B200, operands in DRAM, before (large kernel with 256-column tiles) and now: bf16
 // 16 x 8192 x 8192 (134 MB of weights) 47.5 -> 26.5 us, 128 x 8192 x 8192 49.0 -> 34.2 us; SwiGLU 16 x 3584 x 8192 69.0 ->
 // 26.2 us; fp8 64 x 7168 x 8192 49.2 -> 18.6 us.
-// One MMA holds 128 rows; more of them come in several blocks where that pays (skinny_plan_rows). On both sides of the line at 128 rows, this kernel / the large one with the
-// narrower tiles it now has, L2 flushed, event times in steps of 2 us: bf16 N 8192, K 8192 40.9 / 53.2, K 2048 20.5 / 20.7,
-// K 512 15.7 / 14.6; N 2048, K 1024 16.3 / 14.5 (K up to 1024 is where the large one is level or up to 2 us ahead); SwiGLU N
-// 8192, K 2048 37 / 50; fp8 N 8192, K 2048 19 / 26, N 28672, K 512 22.3 / 20.6.
+// One MMA holds 128 rows; more of them come in several blocks where that pays (skinny_plan_rows). On both sides of the line at
+// 128 rows, this kernel / the large one with the narrower tiles it now has, L2 flushed, event times in steps of 2 us: bf16 N 8192,
+// K 8192 40.9 / 53.2, K 2048 20.5 / 20.7, K 512 15.7 / 14.6; N 2048, K 1024 16.3 / 14.5 (K up to 1024 is where the large one is level
+// or up to 2 us ahead); SwiGLU N 8192, K 2048 37 / 50; fp8 N 8192, K 2048 19 / 26, N 28672, K 512 22.3 / 20.6.
 //
 //   warp 0     TMA producer: weights (streamed, evict first) and activations (kept in L2) of a K block per stage
 //   warp 1     MMA issuer, accumulators in tensor memory: lane = weight row, column = token
