@@ -142,6 +142,22 @@ __device__ __forceinline__ bool wait_counter(const uint32_t *ctr, uint32_t targe
     }
 }
 
+// nvl::ld_nc16 where `on`. Predicated: a branch around the load would make the warp wait for each load before it issues the next one.
+__device__ __forceinline__ uint4 ld_nc16_if(const void *p, bool on)
+{
+    uint4 v = make_uint4(0, 0, 0, 0);
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "setp.ne.u32 q, %5, 0;\n"
+        "@q ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+        "}\n"
+        : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+        : "l"(p), "r"((uint32_t)on)
+        : "memory");
+    return v;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
 {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -151,8 +167,9 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
 // "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): as exact as the guarded division but for
 // about one value in a million that lies on a rounding boundary, and without that division's branch, which made the values of a
 // thread wait for one another, about 150 cycles each (276 x 2 x 640 x 512 20.7 us, now 10.4; 4096 x 2 x 1024 x 512 28.9 and 17.2).
-// Below -87 the divisor would leave the range of the reciprocal and 1 + exp(x) is 1: there the value is x exp(x), with the exponential 2^64 times as large until the last product, so that it is no
-// subnormal number. A divisor of 1 returns the value above it, infinity included.
+// Below -87 the divisor would leave the range of the reciprocal and 1 + exp(x) is 1: there the value is x exp(x), with the
+// exponential 2^64 times as large until the last product, so that it is no subnormal number. A divisor of 1 returns the value
+// above it, infinity included.
 __device__ __forceinline__ float silu(float x)
 {
     constexpr float kLog2e = 1.44269504f;
@@ -470,25 +487,47 @@ __device__ void copier_warps_loop(const GemmParams &p, int rank, int local, int 
     auto copy_all = [&](size_t first, uint32_t cnt, size_t bytes_per_blk, bool scales, bool announce_blocks) {
         const uint32_t total = (uint32_t)n_blocks * cnt;
         int            announced = 0;
-        for (uint32_t j0 = 0; j0 < total && ok; j0 += kCopierThreads * kU) {
-            uint4 v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; u++) {
-                // unconditional (past the end the last item again): behind a branch a load would wait for the one before it
-                const uint32_t j = min(j0 + (uint32_t)u * kCopierThreads + (uint32_t)tid, total - 1);
-                const uint32_t b = j / cnt, i = j - b * cnt;
-                const int      blk = blk_of((int)b);
-                const char    *src = reinterpret_cast<const char *>(scales ? (const void *)p.sg[blk / mbs] : (const void *)p.xg[blk / mbs]);
-                v[u] = nvl::ld_nc16(src + (size_t)blk * bytes_per_blk + (first + i) * 16);
+        // Where a thread stands: pack i of row block r of shard s. Stepped and not divided, and no step beyond the last item: one
+        // warp issues all of a CTA's loads in fp8, so its own instructions count (fp8 allgather of two ranks, with two warps of
+        // half the loads / one that divides, and loads the last item again past the end / now: 256 x 1024 x 2048 27.0 / 33.7 / 27.3
+        // us, 256 x 7424 x 5376 71.9 / 80.3 / 69.2, 1024 x 2048 x 4096 45.9 / 47.1 / 40.4, 2048 x 8192 x 7168 317 / 265 / 251).
+        struct At {
+            uint32_t i;
+            int      r, s;
+        };
+        auto step = [&](At &at, uint32_t by) {
+            at.i += by;
+            while (at.i >= cnt) {
+                at.i -= cnt;
+                if (++at.r == mbs) {
+                    at.r = 0;
+                    if (++at.s == p.tp_size) at.s = 0;
+                }
             }
+        };
+        At at{0, 0, (rank + 1) % p.tp_size};
+        step(at, (uint32_t)tid);
+        for (uint32_t j0 = 0; j0 < total && ok; j0 += kCopierThreads * kU) {
+            uint4    v[kU];
+            At       to = at;
+            uint32_t j  = j0 + (uint32_t)tid;
 #pragma unroll
             for (int u = 0; u < kU; u++) {
-                const uint32_t j = j0 + (uint32_t)u * kCopierThreads + (uint32_t)tid;
+                if (j0 + (uint32_t)u * kCopierThreads < total) {   // the same for all
+                    const char *src = reinterpret_cast<const char *>(scales ? (const void *)p.sg[at.s] : (const void *)p.xg[at.s]);
+                    v[u] = ld_nc16_if(src + (size_t)(at.s * mbs + at.r) * bytes_per_blk + (first + at.i) * 16, j < total);
+                    step(at, kCopierThreads);
+                    j += kCopierThreads;
+                }
+            }
+            j = j0 + (uint32_t)tid;
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
                 if (j < total) {
-                    const uint32_t b = j / cnt, i = j - b * cnt;
-                    const int      blk = blk_of((int)b);
-                    char          *dst = reinterpret_cast<char *>(scales ? (void *)p.sg[rank] : (void *)p.xg[rank]);
-                    *reinterpret_cast<uint4 *>(dst + (size_t)blk * bytes_per_blk + (first + i) * 16) = v[u];
+                    char *dst = reinterpret_cast<char *>(scales ? (void *)p.sg[rank] : (void *)p.xg[rank]);
+                    *reinterpret_cast<uint4 *>(dst + (size_t)(to.s * mbs + to.r) * bytes_per_blk + (first + to.i) * 16) = v[u];
+                    step(to, kCopierThreads);
+                    j += kCopierThreads;
                 }
             }
             ok = sync_all_well();

@@ -1293,3 +1293,35 @@ def test_gemm_fp8_blockscaled_many_tiles_per_walker(dev, M, N, K_, off):
     # half a unit in the last place of bf16 (2^-9), and 32-bit sums of K products far below the largest value of the row
     assert bool(((guard[1:M + 1].double() - want).abs() <= 2 ** -8 * want.abs() + 2e-5 * want.abs().amax(-1, keepdim=True)).all())
     assert bool((guard[0] == 7).all()) and bool((guard[M + 1] == 7).all())
+
+
+_COPIER_SCRIPT = r"""
+import torch
+from xccl_b200.models.tp_mlp import TpMlp, TpMlpFp8, reference_forward_fp32
+from xccl_b200.ops import gemm
+g = torch.Generator(device="cuda").manual_seed(4)
+for fp8, hidden in ((False, 8), (False, 136), (False, 2056), (True, 128), (True, 384), (True, 2176)):
+    for tp, tokens in ((2, 256), (2, 1280), (4, 1536), (3, 384)):
+        mlp = (TpMlpFp8 if fp8 else TpMlp)(tokens, hidden, 256 * tp, tp=tp)
+        x = torch.randn(tokens, hidden, device="cuda", generator=g).to(torch.bfloat16)
+        for _ in range(2):
+            x = x.roll(1, 0)
+            y = torch.cat(mlp.forward(list(x.chunk(tp, 0))), 0).float()
+            mlp.check_error()
+        want = reference_forward_fp32(x, torch.cat(mlp.w_gate, 0), torch.cat(mlp.w_up, 0), torch.cat(mlp.w_down, 1))
+        # bf16: two roundings and one of every rank's partial sum; fp8: 2^-4 per quantised operand, averaged over the sums
+        assert float((y - want).abs().max()) <= (0.08 if fp8 else 0.02) * float(want.abs().max()) + 1e-3, (fp8, hidden, tp, tokens)
+        mlp.close()
+print("copiers ok")
+"""
+
+
+def test_tp_mlp_copier_warps_over_blocks_and_shards(dev):
+    """Copier warps (asked for on more ranks than they are chosen for): shares of a row block from none and one pack to several
+    batches, several row blocks and shards, a last batch that is not full."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    env = dict(os.environ, PYTHONPATH=str(Path(__file__).resolve().parent.parent), XCCL_TP_COPY_MODE="1")
+    r = subprocess.run([sys.executable, "-c", _COPIER_SCRIPT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "copiers ok" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
