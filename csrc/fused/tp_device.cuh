@@ -32,7 +32,7 @@ constexpr int      kScaleRing = 4;
 constexpr uint32_t kScaleRingBytes = 2 * kBM * 4;
 // fp8: registers of a thread of the first four warps (loads, MMAs, copier, scales) and of the eight promotion warps, which hold 128
 // running sums and 32 values on their way; twelve warps alike would get 168. Some values still spill (bytes stored / loaded per
-// thread: CTA pairs 100 / 256, single CTAs 144 / 212).
+// thread: CTA pairs 80 / 232, single CTAs 144 / 256).
 constexpr int      kRegsOthers = 104, kRegsPromotion = 200;
 
 struct Tile {

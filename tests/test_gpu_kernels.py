@@ -1199,11 +1199,13 @@ def test_silu_is_as_exact_as_a_rounded_division(dev):
     assert out[0] == float("inf") and out[1] != out[1] and out[2] != out[2] and out[3] == 0
 
 
-@pytest.mark.parametrize("tp,tokens,hidden,ffn", [(2, 2048, 1152, 3840), (2, 2048, 2048, 4096), (4, 2048, 1152, 4608), (4, 2048, 2048, 4096)])
+@pytest.mark.parametrize("tp,tokens,hidden,ffn", [(2, 2048, 1152, 3840), (2, 2048, 2048, 4096), (4, 2048, 1152, 4608), (4, 2048, 2048, 4096),
+                                                   (2, 1024, 1280, 2816), (4, 1024, 1408, 3072), (2, 256, 1664, 2048)])
 def test_tp_mlp_fp8_walkers_of_local_and_gathered_tiles(dev, tp, tokens, hidden, ffn):
     """The fp8 block over emulated ranks with three to four tiles for every walker, local rows first and gathered rows after
     them: scales that differ strongly from row to row and from K block to K block reach the right tile, and those of gathered
-    rows are read when they have arrived. K in groups of four blocks (16-byte scale loads) and not."""
+    rows are read when they have arrived. K in groups of four blocks (16-byte scale loads) and every remainder; the last three
+    sizes have a tile or two per walker, of single CTAs in the very last."""
     from xccl_b200.models.tp_mlp import TpMlpFp8
     from xccl_b200.ops import gemm
     mlp = TpMlpFp8(tokens, hidden, ffn, tp=tp, emulate=True, fuse_quant=False)
